@@ -809,7 +809,7 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
     }
   } else if (warp == kMmaWarp) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       uint32_t stage = 0, fph = 0;
       bool issued = false;
@@ -1268,7 +1268,7 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
           if (t_next >= 0) load_mask_words(A, t_next / A.n_tiles, lane, w);
           nch = __popc(tmk.tm) * P.cpo;
         }
-        if (lane == 0) {
+        if (elect_one()) {
           const int ab = it & 1;
           const uint32_t aph = (it >> 1) & 1;
           if (!mbar_wait(&acc_empty[ab], aph ^ 1u, abort_flag)) {
@@ -1315,10 +1315,10 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
             }
           }
         }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok || !have) break;
       }
-      if (lane == 0 && issued) {
+      if (issued) {  // the elected lane's
         // no tcgen05.mma may be in flight when TMEM is released
         mma_commit(drain_bar);
         int never = 0;

@@ -712,7 +712,7 @@ __global__ void __maxnreg__(kPair ? 80 : 96) conv_wgrad_kernel(const __grid_cons
     }
   } else if (warp == kMmaWarp) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       // stage, full phase, dOut buffer and its phase of the ring of the
       // current chunk (c) and of the other ring (o); the rings alternate

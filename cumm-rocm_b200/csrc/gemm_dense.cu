@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
 
   if (warp == 4) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, eph = 0;
       bool ok = true;
       for (int64_t u = blockIdx.x; u < P.units && ok; u += gridDim.x) {
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
     }
   } else if (warp == 5) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, fph = 0;
       bool issued = false, ok = true;
       int it = 0;
