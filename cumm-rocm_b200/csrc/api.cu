@@ -454,7 +454,7 @@ int sc_conv_implicit_gemm(const sc_conv_params *p) {
     const int64_t own = own_sorted_bytes(p, es);
     if (own > 0 && ws != nullptr && p->workspace_bytes >= plan.ws_bytes) {
       int32_t *tab = reinterpret_cast<int32_t *>(ws + plan.ws_bytes - own);
-      e = scb::sort_indices(p->indices, p->kv, p->N, p->mask_argsort, tab, s);
+      e = scb::sort_indices(p->indices, p->kv, p->N, p->mask_argsort, nullptr, 0, tab, s);
       if (e != cudaSuccess) return cuda_fail(e, "sorted index table");
       a.idx_sorted = tab;
     }
@@ -801,10 +801,12 @@ int sc_build_conv_outputs(const int32_t *coords, int64_t n_in, int32_t batch, co
   rc = device_state(&a.err, &sms);
   if (rc != SC_OK) return rc;
   for (int d = 0; d < 3; ++d) out_spatial[d] = a.out_spatial[d];
-  cudaError_t e = scb::build_conv_outputs(a, n_out, workspace, workspace_bytes,
+  int bits = 0;
+  cudaError_t e = scb::build_conv_outputs(a, n_out, &bits, workspace, workspace_bytes,
                                           static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "build_conv_outputs");
-  return sync_check(static_cast<cudaStream_t>(stream));
+  // the word came with the output count; only an error is worth its own round trip
+  return bits ? sync_check(static_cast<cudaStream_t>(stream)) : SC_OK;
 }
 
 int sc_build_conv_pairs(const int32_t *coords, int64_t n_in, int32_t batch, const int32_t *spatial,
@@ -833,11 +835,16 @@ int sc_build_conv_pairs(const int32_t *coords, int64_t n_in, int32_t batch, cons
 
 int sc_sort_indices(const int32_t *indices, int32_t kv, int64_t N, const int32_t *argsort,
                     int32_t *indices_sorted, void *stream) {
+  return sc_sort_indices_masked(indices, kv, N, argsort, nullptr, 0, indices_sorted, stream);
+}
+
+int sc_sort_indices_masked(const int32_t *indices, int32_t kv, int64_t N, const int32_t *argsort,
+                           const uint32_t *mask, int32_t reverse, int32_t *indices_sorted, void *stream) {
   g_last_error.clear();
   if (N > 0 && (indices == nullptr || argsort == nullptr || indices_sorted == nullptr))
     return fail(SC_INVALID_ARG, "null indices / argsort / output");
   if (kv < 1 || kv > 32 || N < 0) return fail(SC_INVALID_ARG, "bad kv / N");
-  cudaError_t e = scb::sort_indices(indices, kv, N, argsort, indices_sorted,
+  cudaError_t e = scb::sort_indices(indices, kv, N, argsort, mask, reverse ? 1 : 0, indices_sorted,
                                     static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_fail(e, "sort_indices");
   return SC_OK;

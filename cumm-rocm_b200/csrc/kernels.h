@@ -202,14 +202,17 @@ struct PairBuildArgs {
 int64_t pairs_workspace_bytes(int64_t n_in, int kv, int subm);
 cudaError_t build_subm_pairs(const PairBuildArgs &a, int32_t *pairs_fwd, int32_t *pairs_bwd,
                              uint32_t *mask_fwd, void *ws, int64_t ws_bytes, cudaStream_t s);
-cudaError_t build_conv_outputs(const PairBuildArgs &a, int64_t *n_out, void *ws,
+// err_bits: the device error word as of this build (not cleared)
+cudaError_t build_conv_outputs(const PairBuildArgs &a, int64_t *n_out, int *err_bits, void *ws,
                                int64_t ws_bytes, cudaStream_t s);
 cudaError_t build_conv_pairs(const PairBuildArgs &a, int64_t n_out, int32_t *out_coords,
                              int32_t *pairs_fwd, int32_t *pairs_bwd, uint32_t *mask_fwd,
                              uint32_t *mask_bwd, void *ws, int64_t ws_bytes, cudaStream_t s);
 int64_t sort_workspace_bytes(int64_t n);
+// mask: null, or the sorted masks (bit k, of the kv-bit reversed word with
+// `reverse`, clear: indices[k][argsort[r]] is -1 and is not read)
 cudaError_t sort_indices(const int32_t *indices, int kv, int64_t n, const int32_t *argsort,
-                         int32_t *out, cudaStream_t s);
+                         const uint32_t *mask, int reverse, int32_t *out, cudaStream_t s);
 cudaError_t sort_masks_split(uint32_t *data, int64_t n, uint32_t split_mask, int32_t *argsort,
                              void *ws, int64_t ws_bytes, cudaStream_t s);
 

@@ -21,6 +21,7 @@ EXPORTS = (
     "sc_pairs_workspace_size", "sc_build_subm_pairs", "sc_build_conv_outputs",
     "sc_build_conv_pairs", "sc_sort_masks_split", "sc_sort_workspace_size",
     "sc_check_device_error", "sc_last_error", "sc_version", "sc_sort_indices",
+    "sc_sort_indices_masked",
     "sc_conv_wgrad_static_scratch", "sc_gather_rows", "sc_scatter_add_rows",
     "sc_tile_order", "sc_tile_order_workspace_size",
 )
@@ -94,6 +95,7 @@ def load() -> ctypes.CDLL:
         lib.sc_sort_workspace_size.argtypes = [c_i64, P(c_i64)]
         lib.sc_check_device_error.argtypes = [c_vp, P(c_i32)]
         lib.sc_sort_indices.argtypes = [c_vp, c_i32, c_i64, c_vp, c_vp, c_vp]
+        lib.sc_sort_indices_masked.argtypes = [c_vp, c_i32, c_i64, c_vp, c_vp, c_i32, c_vp, c_vp]
         lib.sc_tile_order_workspace_size.argtypes = [c_i64, P(c_i64)]
         lib.sc_tile_order.argtypes = [c_vp, c_i64, c_u32, c_i32, c_i32, c_vp, c_vp, c_i64, c_vp]
         lib.sc_gather_rows.argtypes = [c_vp, c_vp, c_i64, c_vp, c_i64, c_i64, c_i32, c_i32, c_vp]

@@ -76,14 +76,17 @@ class SpconvOps:
         _lib.check(lib.sc_pairs_workspace_size(n, kv, 1, ctypes.byref(need)))
         ws = _ws(need.value, dev)
         sp, ks, dl = _i32x3(spatial_shape), _i32x3(ksize), _i32x3(dilation)
-        mask_full = torch.empty(n, dtype=torch.int32, device=dev)
+        # without a split the kernel writes the caller's mask row itself
+        direct = split_masks is None and masks.dtype == torch.int32 and masks[0].is_contiguous()
+        mask_full = masks[0] if direct else torch.empty(n, dtype=torch.int32, device=dev)
         s = _stream(stream)
         _lib.check(lib.sc_build_subm_pairs(
             _vp(coords), n, ctypes.c_void_p(sp.data_ptr()), ctypes.c_void_p(ks.data_ptr()),
             ctypes.c_void_p(dl.data_ptr()), _vp(pairs[0]), _vp(pairs[1]), _vp(mask_full), _vp(ws),
             ws.numel(), s))
         if split_masks is None:
-            masks[0].copy_(mask_full)
+            if not direct:
+                masks[0].copy_(mask_full)
         else:
             for j, sm in enumerate(split_masks):
                 masks[j].copy_(mask_full & _as_i32(sm))
@@ -158,15 +161,19 @@ class SpconvOps:
         return SpconvOps.sort_1d_by_key_split(data, 0xffffffff, stream)
 
     @staticmethod
-    def sort_indices(indices, argsort, stream: int = 0):
+    def sort_indices(indices, argsort, stream: int = 0, mask=None, reverse: bool = False):
         """indices [kv, N] permuted into argsort order: out[k][r] =
-        indices[k][argsort[r]] (the optional ConvParams.indices_sorted)."""
+        indices[k][argsort[r]] (the optional ConvParams.indices_sorted).
+        ``mask``: the sorted masks [N], bit k (of the kv-bit reversed word with
+        ``reverse``) set exactly where out[k][r] != -1; absent entries are then
+        not read."""
         _lib.require_cuda()
         lib = _lib.load()
         ind, srt = _t(indices), _t(argsort)
         kv, n = ind.shape
         out = torch.empty_like(ind)
-        _lib.check(lib.sc_sort_indices(_vp(ind), kv, n, _vp(srt), _vp(out), _stream(stream)))
+        _lib.check(lib.sc_sort_indices_masked(_vp(ind), kv, n, _vp(srt), _vp(_t(mask)), 1 if reverse else 0,
+                                              _vp(out), _stream(stream)))
         if isinstance(indices, tv.Tensor):
             return tv.Tensor(out, tv.int32)
         return out
@@ -230,11 +237,16 @@ class PairTable:
         cache = self.__dict__.setdefault("_sorted_cache", {})
         key = (which, split)
         if key not in cache:
+            # the masks of the rows say which entries exist
             if which == "fwd":
-                cache[key] = SpconvOps.sort_indices(self.pairs_fwd, self.argsorts_fwd[split])
+                cache[key] = SpconvOps.sort_indices(self.pairs_fwd, self.argsorts_fwd[split],
+                                                    mask=self.masks_fwd[split])
+            elif self.subm:
+                cache[key] = SpconvOps.sort_indices(self.pairs_bwd, self.argsorts_fwd[split],
+                                                    mask=self.masks_fwd[split], reverse=True)
             else:
-                order = self.argsorts_fwd[split] if self.subm else self.argsorts_bwd[split]
-                cache[key] = SpconvOps.sort_indices(self.pairs_bwd, order)
+                cache[key] = SpconvOps.sort_indices(self.pairs_bwd, self.argsorts_bwd[split],
+                                                    mask=self.masks_bwd[split])
         return cache[key]
 
     def tile_order(self, which: str = "fwd", split: int = 0) -> torch.Tensor:
@@ -250,6 +262,18 @@ class PairTable:
             cache[key] = SpconvOps.tile_order(masks[split], self.kv, self.split_masks[split]
                                               if self.split_masks else 0xffffffff)
         return cache[key]
+
+
+def _sorted_masks(mask: torch.Tensor, splits: Sequence[int], kv: int, stream: int):
+    """Per split: the masks sorted by their split bits, and the argsort.  `mask`
+    itself is sorted for the last split.  Bits past kv are never set, so the
+    sort skips their digits."""
+    masks, sorts = [], []
+    for j, sm in enumerate(splits):
+        mm = mask if j == len(splits) - 1 else mask.clone()
+        sorts.append(SpconvOps.sort_1d_by_key_split(mm, sm & ((1 << kv) - 1), stream))
+        masks.append(mm)
+    return masks, sorts
 
 
 def build_pair_table(coords: torch.Tensor, spatial_shape: Sequence[int], ksize=(3, 3, 3),
@@ -273,22 +297,12 @@ def build_pair_table(coords: torch.Tensor, spatial_shape: Sequence[int], ksize=(
         m = torch.empty((1, n), dtype=torch.int32, device=dev)
         SpconvOps.generate_subm_conv_inds(coords, pairs, m, spatial_shape, ksize, dilation,
                                           stream=stream)
-        masks, sorts = [], []
-        for sm in splits:
-            mm = m[0].clone()
-            sorts.append(SpconvOps.sort_1d_by_key_split(mm, sm, stream))
-            masks.append(mm)
+        masks, sorts = _sorted_masks(m[0], splits, kv, stream)
         return PairTable(n, n, kv, True, pairs[0], pairs[1], masks, sorts, split_masks=splits,
                          out_inds=coords, out_spatial=list(spatial_shape))
     out_inds, pf, pb, mf, mb, out_sp = SpconvOps.generate_conv_inds(
         coords, batch_size, spatial_shape, ksize, stride, padding, dilation, stream)
-    masks, sorts, masks_b, sorts_b = [], [], [], []
-    for sm in splits:
-        mm = mf.clone()
-        sorts.append(SpconvOps.sort_1d_by_key_split(mm, sm, stream))
-        masks.append(mm)
-        mb2 = mb.clone()
-        sorts_b.append(SpconvOps.sort_1d_by_key_split(mb2, sm, stream))
-        masks_b.append(mb2)
+    masks, sorts = _sorted_masks(mf, splits, kv, stream)
+    masks_b, sorts_b = _sorted_masks(mb, splits, kv, stream)
     return PairTable(n, out_inds.shape[0], kv, False, pf, pb, masks, sorts, masks_b, sorts_b,
                      splits, out_inds, out_sp)

@@ -274,6 +274,13 @@ int sc_sort_workspace_size(int64_t n, int64_t *bytes);
  * that is reused by several convolutions). */
 int sc_sort_indices(const int32_t *indices, int32_t kv, int64_t N, const int32_t *argsort,
                     int32_t *indices_sorted, void *stream);
+/* The same with the sorted masks of the rows at hand ([N] uint32, bit k set
+ * exactly where indices[k][argsort[r]] != -1; reverse = 1: the kv-bit reversed
+ * word says so, as for submanifold pairs_bwd): absent entries are written as
+ * -1 without being read.  mask may be NULL. */
+int sc_sort_indices_masked(const int32_t *indices, int32_t kv, int64_t N, const int32_t *argsort,
+                           const uint32_t *mask, int32_t reverse, int32_t *indices_sorted,
+                           void *stream);
 
 /* Largest-first tile order for sc_conv_params.tile_order: the 128-row tiles
  * of the mask-sorted rows ordered by the number of offsets they visit
