@@ -21,8 +21,9 @@
 // counter so CTAs that drew small tiles come back for more):
 //   epilogue warps   TMEM -> registers -> act(alpha acc + beta src) -> row
 //                    mask_argsort[r] (permuted store)
-//   producer warps   A rows of each (offset, 128-byte column block) chunk by
-//                    TMA tile::gather4 (4 rows per lane, SWIZZLE_128B or
+//   producer warps   (in groups that take the chunks in turn) A rows of each
+//                    (offset, 128-byte column block) chunk by TMA
+//                    tile::gather4 (4 rows per lane, SWIZZLE_128B or
 //                    SWIZZLE_64B by address; index -1 reads as zero rows, each
 //                    group of 4 gated by its 32-row sub-tile mask) and the
 //                    weight slab by 2-D TMA boxes (backward-input: the [K, kv,
@@ -37,9 +38,8 @@
 //   MMA warp         TMEM allocator + single-thread tcgen05.mma issuer into a
 //                    double-buffered fp32 TMEM accumulator (128 lanes x BN)
 // Layouts (Layout<kPair>): one 17-warp CTA per SM, or on the gather path two
-// 11-warp CTAs per SM (4 producers, 2 loaders): measured on B200 the TMA
-// gather rate is per issuing CTA, so two CTAs per SM gather ~1.5x the rows
-// per cycle, which the kernel, bound by that rate, turns into ~12 % less time.
+// 11-warp CTAs per SM (4 producers, 2 loaders): the gather rate goes with the
+// warps that issue and the stages they can fill.
 // Every mbarrier wait is bounded (globaltimer) and raises a CTA abort flag
 // plus kErrWaitTimeout instead of spinning forever.
 #include <cuda.h>
@@ -83,7 +83,7 @@ struct Meta {
 };
 
 struct KParams {
-  CUtensorMap tmap_a;  // gathered rows [a_rows, red] (TMA path)
+  CUtensorMap tmap_a;  // gathered rows [a_rows, red] (single layout)
   CUtensorMap tmap_b;  // B rows [n_total, kv * red] (TMA path)
   // four rows of zeros with tmap_a's box and swizzle: a gather whose four
   // rows are all -1 reads these instead (out-of-range gather rows cost the
@@ -96,6 +96,7 @@ struct KParams {
   int opc;            // offsets packed per chunk (a_row_bytes < 128)
   int upo;            // 16-byte units per packed offset segment
   int stages;
+  int group_warps;    // gather path: producer warps per chunk
   uint32_t stage_bytes;
   uint32_t b_off;
   uint32_t idx_off;
@@ -143,8 +144,7 @@ __global__ void __launch_bounds__(kOrderWarps * 32)
       const int64_t rq = t * kTileM + q * 32 + lane;
       if (rq < M) v |= mask ? __ldg(mask + rq) : 1u;
     }
-#pragma unroll
-    for (int sh = 16; sh > 0; sh >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, sh);
+    v = __reduce_or_sync(0xffffffffu, v);
     uint32_t tm = v & filter;
     if (reverse) tm = __brev(tm) >> (32 - kv);
     if (lane == 0) {
@@ -262,35 +262,52 @@ __device__ __forceinline__ void store_row(TOut *p, const float *v) {
   }
 }
 
+// The activation of n values.  One branch on the type for all of them: with the
+// switch inside the loop every element branched, 2,100 cycles per 16 columns of
+// a tile and more than half of the epilogue warps' time.
+template <int n>
+__device__ __forceinline__ void apply_act_n(float *v, int type, float a) {
+  if (type == 0) return;
+  if (type == 1) {
+#pragma unroll
+    for (int i = 0; i < n; ++i) v[i] = apply_act(v[i], 1, a);
+  } else if (type == 2) {
+#pragma unroll
+    for (int i = 0; i < n; ++i) v[i] = apply_act(v[i], 2, a);
+  } else if (type == 3) {
+#pragma unroll
+    for (int i = 0; i < n; ++i) v[i] = apply_act(v[i], 3, a);
+  }
+}
+
 // Applies the epilogue to `n` (16 or 32) consecutive columns starting at column
 // `col` of output row `orow` and stores them.
 template <int n, typename TOut>
 __device__ __forceinline__ void epilogue_cols(const KParams &P, float *acc, int64_t orow, int col) {
   const EpiParams &e = P.a.epi;
-  float src[n];
   const bool use_src = e.beta != 0.f && e.src != nullptr;
-  if (use_src) {
-    const TOut *s = reinterpret_cast<const TOut *>(e.src) + orow * e.src_ld + col;
-    load_src<n, TOut>(s, src);
-  }
   if (e.mode == 1) {
-    float bias[n];
-    if (e.bias != nullptr) load_src<n, TOut>(reinterpret_cast<const TOut *>(e.bias) + col, bias);
+    if (e.scale != nullptr) {
 #pragma unroll
-    for (int i = 0; i < n; ++i) {
-      float sc = e.scale != nullptr ? __ldg(e.scale + col + i) : 1.f;
-      float v = sc * acc[i] + (e.bias != nullptr ? e.alpha * bias[i] : 0.f);
-      if (use_src) v = fmaf(e.beta, src[i], v);
-      acc[i] = apply_act(v, e.act_type, e.act_alpha);
+      for (int i = 0; i < n; ++i) acc[i] = __ldg(e.scale + col + i) * acc[i];
+    }
+    if (e.bias != nullptr) {
+      float bias[n];
+      load_src<n, TOut>(reinterpret_cast<const TOut *>(e.bias) + col, bias);
+#pragma unroll
+      for (int i = 0; i < n; ++i) acc[i] = acc[i] + e.alpha * bias[i];
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < n; ++i) {
-      float v = e.alpha * acc[i];
-      if (use_src) v = fmaf(e.beta, src[i], v);
-      acc[i] = apply_act(v, e.act_type, e.act_alpha);
-    }
+    for (int i = 0; i < n; ++i) acc[i] = e.alpha * acc[i];
   }
+  if (use_src) {
+    float src[n];
+    load_src<n, TOut>(reinterpret_cast<const TOut *>(e.src) + orow * e.src_ld + col, src);
+#pragma unroll
+    for (int i = 0; i < n; ++i) acc[i] = fmaf(e.beta, src[i], acc[i]);
+  }
+  apply_act_n<n>(acc, e.act_type, e.act_alpha);
   TOut *dst = reinterpret_cast<TOut *>(P.a.out) + orow * P.a.out_ld + col;
   store_row<n, TOut>(dst, acc);
 }
@@ -368,10 +385,10 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S; ++i) {
-      // gather: one arrive.expect_tx per producer warp; cp.async: the 32
+      // gather: one arrive per warp of the stage's group; cp.async: the 32
       // lanes of the stage's producer warp (cp.async.mbarrier.arrive.noinc)
       // plus, with TMA, one arrive.expect_tx for the weight slab
-      mbar_init(&full_bar[i], kGather ? kProdWarps : 32 + (kTma ? 1 : 0));
+      mbar_init(&full_bar[i], kGather ? P.group_warps : 32 + (kTma ? 1 : 0));
       mbar_init(&empty_bar[i], 1);
     }
     for (int i = 0; i < kIdxStages; ++i) {
@@ -508,8 +525,7 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
           for (int q = 0; q < 4; ++q) {
             const int64_t rq = tile_m * kTileM + q * 32 + lane;
             uint32_t v = rq < A.M ? (A.mask ? __ldg(A.mask + rq) : 1u) : 0u;
-#pragma unroll
-            for (int sh = 16; sh > 0; sh >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, sh);
+    v = __reduce_or_sync(0xffffffffu, v);
             gq[q] = v;
           }
           g0 = gq[0];
@@ -591,24 +607,31 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
     // ---------------------------------------------------------------- producers
     const int pw = warp - kProdWarp0;
     if constexpr (kGather) {
-    // TMA gather: all kProdWarps warps serve every chunk; lanes 0-3 of warp pw
-    // each issue one tile::gather4 (4 rows x 128 bytes, SWIZZLE_128B by
-    // address) for rows [16 pw, 16 pw + 16) of the stage.  An index of -1 is
-    // an out-of-range row and lands as zeros.  Lane 0 of every warp arrives
-    // with expect_tx for its 2 KB (one warp in turn adds the weight slab), so
-    // a stage completes on kProdWarps arrivals plus the copied bytes.  Every
-    // warp arrives once per use of stage s and empty phase n cannot complete
-    // before all of them did, so no warp runs two phases ahead of a wait.
-    // (Measured on B200: 8 warps of gather4 fill a 16 KB stage in ~740
-    // cycles; per-thread cp.async arrivals serialise on the barrier word.)
+    // Groups of P.group_warps warps take the chunks in turn, each warp an equal
+    // share of the rows: a chunk costs a warp a fixed ~1,000 cycles of waits and
+    // set-up beside its rows, so fewer warps per chunk and more chunks in
+    // flight fill the ring faster.  There are at most as many groups as
+    // stages: a group that tests stage s then knows the use before the last
+    // one to be consumed, which the parity test needs.
+    // TMA tile::gather4, one lane per four rows (an index of -1 is an
+    // out-of-range row and lands as zeros): about 130 cycles of a warp's issue
+    // each, asynchronous from there.  With all producer warps on every chunk,
+    // against two: 60k voxels C = K = 128 forward 94 -> 62 us, C = K = 256
+    // 191 -> 154; 200k voxels, stride 2, E4M3 64 -> 128 47 -> 39.  16-byte
+    // cp.async copies by the same groups: as fast for 64-byte rows, slower for
+    // 128-byte ones (114 us at C = K = 128).
     const int esz = kF8 ? 1 : 2;
     const int rb = P.row_bytes;  // 128, or 64 for 64-byte rows (SWIZZLE_64B stages)
     const int box = rb / esz;
-    const uint32_t a_tx = (kTileM / kProdWarps) * static_cast<uint32_t>(rb);
+    const int W = P.group_warps;
+    const int groups = kProdWarps / W;
+    const int grp = pw / W;
+    const int rows = kTileM / W;           // per warp
+    const int r_base = (pw - grp * W) * rows;
     const uint32_t b_tx = static_cast<uint32_t>(A.BN) * rb;
-    const int r0 = pw * (kTileM / kProdWarps) + lane * 4;
     int it = 0;
-    uint32_t stage = 0, eph = 0, gchunk = 0;
+    uint32_t stage = 0, eph = 0;
+    int turn = 0;                          // chunk % groups
     bool ok = true;
     for (; ok; ++it) {
       const int b = it % kIdxStages;
@@ -625,52 +648,49 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
       const int nch = meta->nchunks;
       const int n0 = (tile % A.n_tiles) * A.BN;
       for (int j = 0; j < nch; ++j) {
-        const uint32_t s = stage;
-        const int slot_a = j / P.cpo;
-        const int cb = j - slot_a * P.cpo;
-        const int k = meta->k_list[slot_a];
-        const uint32_t sA = smem_base + s * P.stage_bytes;
-        if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], eph ^ 1, abort_flag))) {
-          if (lane == 0) flag_error(A.err, kErrWaitTimeout);
-          ok = false;
-          break;
-        }
-        if (lane == 0) {
-          if (static_cast<int>(gchunk % kProdWarps) == pw) {
-            mbar_arrive_expect_tx(&full_bar[s], a_tx + b_tx);
+        if (turn == grp) {
+          const int slot_a = P.cpo == 1 ? j : j / P.cpo;
+          const int cb = j - slot_a * P.cpo;
+          const int k = meta->k_list[slot_a];
+          const uint32_t sA = smem_base + stage * P.stage_bytes;
+          if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[stage], eph ^ 1u, abort_flag))) {
+            if (lane == 0) flag_error(A.err, kErrWaitTimeout);
+            ok = false;
+            break;
+          }
+          if (lane == 0) mbar_arrive_expect_tx(&full_bar[stage], rows * rb + (r_base == 0 ? b_tx : 0u));
+          __syncwarp();
+          if (r_base == 0 && elect_one()) {
             if (P.b_mn) {
               // rows j = cb * 64 .. + 63 of the weight, columns k * C + n0 + 64 q
               for (int q = 0; q < A.BN / 64; ++q)
                 tma_load_2d(sA + P.b_off + q * 8192, &P.tmap_b, k * (A.b_off_stride / esz) + n0 + 64 * q,
-                            cb * 64, &full_bar[s]);
+                            cb * 64, &full_bar[stage]);
             } else {
-              tma_load_2d(sA + P.b_off, &P.tmap_b, k * (A.b_off_stride / esz) + cb * box, n0,
-                          &full_bar[s]);
+              tma_load_2d(sA + P.b_off, &P.tmap_b, k * (A.b_off_stride / esz) + cb * box, n0, &full_bar[stage]);
             }
-          } else {
-            mbar_arrive_expect_tx(&full_bar[s], a_tx);
+          }
+          if (lane * 4 < rows) {
+            const int r = r_base + lane * 4;
+            int4 q = *reinterpret_cast<const int4 *>(tab + k * kTileM + r);
+            // rows r .. r + 3 share a 32-row group: gate by its sub-tile mask
+            // (bulk-copied tables are ungated) and check the indices
+            if (!((meta->sub[r >> 5] >> k) & 1u)) q = make_int4(-1, -1, -1, -1);
+            const bool bad = q.x < -1 || q.x >= A.a_rows || q.y < -1 || q.y >= A.a_rows || q.z < -1 ||
+                             q.z >= A.a_rows || q.w < -1 || q.w >= A.a_rows;
+            if (bad) {
+              flag_error(A.err, kErrBadIndex);
+              q = make_int4(-1, -1, -1, -1);
+            }
+            if (P.zero_ok && (q.x & q.y & q.z & q.w) == -1) {
+              const int z = zero_group(blockIdx.x * 128 + pw * 16 + lane, stage + static_cast<uint32_t>(j));
+              tma_gather4(sA + r * rb, &P.tmap_zero, 0, z, z + 1, z + 2, z + 3, &full_bar[stage]);
+            } else {
+              tma_gather4(sA + r * rb, &P.tmap_a, cb * box, q.x, q.y, q.z, q.w, &full_bar[stage]);
+            }
           }
         }
-        __syncwarp();
-        if (lane < (kTileM / kProdWarps) / 4) {
-          int4 q = *reinterpret_cast<const int4 *>(tab + k * kTileM + r0);
-          // rows r0..r0+3 share a 32-row group: gate by its sub-tile mask
-          // (bulk-copied tables are ungated) and check the indices
-          if (!((meta->sub[r0 >> 5] >> k) & 1u)) q = make_int4(-1, -1, -1, -1);
-          const bool bad = q.x < -1 || q.x >= A.a_rows || q.y < -1 || q.y >= A.a_rows ||
-                           q.z < -1 || q.z >= A.a_rows || q.w < -1 || q.w >= A.a_rows;
-          if (bad) {
-            flag_error(A.err, kErrBadIndex);
-            q = make_int4(-1, -1, -1, -1);
-          }
-          if (P.zero_ok && (q.x & q.y & q.z & q.w) == -1) {
-            const int z = zero_group(blockIdx.x * 32 + pw * 8 + lane, gchunk);
-            tma_gather4(sA + r0 * rb, &P.tmap_zero, 0, z, z + 1, z + 2, z + 3, &full_bar[s]);
-          }
-          else
-            tma_gather4(sA + r0 * rb, &P.tmap_a, cb * box, q.x, q.y, q.z, q.w, &full_bar[s]);
-        }
-        ++gchunk;
+        if (++turn == groups) turn = 0;
         if (++stage == static_cast<uint32_t>(S)) {
           stage = 0;
           eph ^= 1u;
@@ -918,8 +938,7 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
         const int64_t rr = tile_m * kTileM + q * 32 + lane;
         if (rr < A.M) km |= A.mask ? __ldg(A.mask + rr) : 1u;
       }
-#pragma unroll
-      for (int s = 16; s > 0; s >>= 1) km |= __shfl_xor_sync(0xffffffffu, km, s);
+      km = __reduce_or_sync(0xffffffffu, km);
       km &= A.mask_filter;
       if (!mbar_wait(&acc_full[ab], aph, abort_flag)) {
         flag_error(A.err, kErrWaitTimeout);
@@ -954,32 +973,41 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
 
 // ------------------------------------------------------------------ strand kernel
 // Forward / backward-input over 128-byte (SWIZZLE_128B) or 64-byte
-// (SWIZZLE_64B: C = 64 e4m3, C = 32 bf16 / f16) gathered rows with several
-// independent pipelines ("strands") per SM: two CTAs per SM, each running
-// kStrands strands.  A strand owns kSProd producer warps, its own ring of
-// P.stages stages (128 gathered rows + the weight slab; as many as fit, 2 of
-// 24 KB for 128-byte rows at BN = 64, 4 of 12 KB for 64-byte rows), one MMA
-// warp and a double-buffered TMEM accumulator; the four epilogue warps of the
-// CTA serve both strands.  The kernel is bound by the latency of its rings
-// (each stage needs a producer -> MMA -> producer round trip), so the ring
-// depth that shared memory allows sets its speed.  Measured on B200: one tcgen05.mma stream (one issuing warp)
-// completes an M = 128, K = 16 MMA about every 170 cycles whatever N is, and
-// one producer ring (its warps, stages and barriers) fills ~18-30 bytes per
-// cycle; both rates grow with the number of independent streams on the SM
-// (four MMA warps: ~5450 FLOP/clk/SM at N = 64; four rings of four TMA warps:
-// ~65 B/clk/SM), which the strands provide.  Tiles are taken in the
-// largest-first order when one is given (strand_tile), else round-robin.  Every role derives its tiles' masks itself (the
-// tile's mask words OR-ed per 32-row group), and the producers read each
-// gather's four indices straight from the sorted index table, so the strands
-// share no index ring.  Needs indices_sorted (16-byte aligned, M % 4 == 0)
-// and BN <= 64.
-constexpr int kStrands = 2;
-constexpr int kSProd = 4;
-constexpr int kSMaxStages = 4;  // stages per strand: 2 of 24 KB (128-byte rows), 4 of 12 KB (64-byte rows)
-constexpr int kSWarps = kEpiWarps + kStrands * (kSProd + 1);  // 14
+// (SWIZZLE_64B: C = 64 e4m3, C = 32 bf16 / f16) gathered rows: two CTAs per
+// SM, each one pipeline ("strand") of kSProd producer warps in groups of
+// kSGroupWarps that take the chunks in turn, a ring of P.stages stages (128
+// gathered rows + the weight slab; as many as fit, 4 of 24 KB for 128-byte rows
+// at BN = 64, 8 of 12 KB for 64-byte rows), one MMA warp, a double-buffered TMEM
+// accumulator and four epilogue warps.
+//
+// What bounds it, from clock64() counters of every role (200k voxels, C = K =
+// 64): not the tensor core (its warp waits) but the time a chunk holds its
+// stage: a gather4 takes ~110 cycles of its warp's issue, so ~1,750 for a
+// warp's 16, then ~900 until the rows have landed, ~700 in the MMAs and ~500
+// until the stage is issued again, over 4 stages.  Hence two warps per chunk
+// and four chunks in flight.  Steps, forward us at 200k voxels / 2.6M voxels /
+// 4k voxels: two strands of two stages with four warps on every chunk (1,800
+// cycles of waits, set-up and issue per chunk and warp) 74 / 781 / 37; epilogue
+// without a branch per element 69 / 777 / 33 (with cp.async gathers instead of
+// gather4 67 / 740 / 31); one strand of four stages with warps in groups 61 /
+// 704 / 16; tile ids and masks loaded two tiles ahead 58 / 674 / 16.  Four
+// warps per chunk: 66 / 732 / 19.  Two accumulators per tile for the MMA chain:
+// no change.
+//
+// Tiles are taken in the largest-first order when one is given (strand_tile),
+// else round-robin.  Every role derives its tiles' masks itself (the tile's
+// mask words OR-ed per 32-row group), and the producers read each gather's four
+// indices straight from the sorted index table, so the roles share no index
+// ring.  Needs indices_sorted (16-byte aligned, M % 4 == 0) and BN <= 64.
+constexpr int kStrands = 1;
+constexpr int kSProd = 8;
+constexpr int kSGroupWarps = 2;                       // producer warps per chunk
+constexpr int kSGroups = kSProd / kSGroupWarps;
+constexpr int kSMaxStages = 8;  // stages per strand: 4 of 24 KB (128-byte rows), 8 of 12 KB (64-byte rows)
+constexpr int kSWarps = kEpiWarps + kStrands * (kSProd + 1);  // 13
 constexpr int kSThreads = kSWarps * 32;
 constexpr int kSBars = 2 * kSMaxStages + 7;  // barriers per strand
-constexpr uint32_t kSTmemCols = 256;      // per CTA: kStrands x 2 buffers x BN (<= 64)
+constexpr uint32_t kSTmemCols = kStrands * 128;  // per CTA: 2 buffers x BN (<= 64) per strand
 
 struct TileMasks {
   uint32_t g[4];    // OR of each 32-row group (unfiltered)
@@ -1002,10 +1030,7 @@ __device__ __forceinline__ TileMasks reduce_masks(const ConvRowGatherArgs &A, co
   TileMasks t;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    uint32_t v = w[q];
-#pragma unroll
-    for (int sh = 16; sh > 0; sh >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, sh);
-    t.g[q] = v;
+    t.g[q] = __reduce_or_sync(0xffffffffu, w[q]);
   }
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -1028,13 +1053,11 @@ __device__ __forceinline__ TileMasks reduce_masks(const ConvRowGatherArgs &A, co
 // (0 .. nstr-1, then nstr-1 .. 0, ...), so the strand that drew the heaviest
 // tile of one round draws the lightest of the next; without it, every nstr-th
 // tile.
-__device__ __forceinline__ int64_t strand_tile(const KParams &P, int64_t pos, int64_t nstr, int64_t it) {
-  if (P.a.tile_order == nullptr) {
-    const int64_t d = it * nstr + pos;
-    return d < P.num_tiles ? d : -1;
-  }
-  const int64_t d = it * nstr + ((it & 1) ? nstr - 1 - pos : pos);
-  return d < P.num_tiles ? scheduled_tile(P.a, d) : -1;
+__device__ __forceinline__ int strand_tile(const KParams &P, int pos, int nstr, int it) {
+  const int n = static_cast<int>(P.num_tiles);
+  const int d = it * nstr + (P.a.tile_order != nullptr && (it & 1) ? nstr - 1 - pos : pos);
+  if (d >= n) return -1;
+  return P.a.tile_order != nullptr ? static_cast<int>(scheduled_tile(P.a, d)) : d;
 }
 
 template <bool kF8, typename TOut, bool kWide>
@@ -1045,9 +1068,9 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
   uint8_t *smem = smem_raw + pad;
   const uint32_t smem_base = raw_u32 + pad;
   const ConvRowGatherArgs &A = P.a;
-  // kWide: 128-byte rows (SWIZZLE_128B), two 24 KB stages per strand; else
-  // 64-byte rows (SWIZZLE_64B), four 12 KB stages
-  constexpr int S = kWide ? 2 : 4;
+  // kWide: 128-byte rows (SWIZZLE_128B), four 24 KB stages per strand; else
+  // 64-byte rows (SWIZZLE_64B), eight 12 KB stages
+  constexpr int S = kWide ? 4 : 8;
   constexpr int rb = kWide ? 128 : 64;
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + P.bar_off);
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kStrands * kSBars);
@@ -1060,7 +1083,7 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
     for (int s = 0; s < kStrands; ++s) {
       uint64_t *b = bars + s * kSBars;
       for (int i = 0; i < S; ++i) {
-        mbar_init(&b[i], kSProd);  // full: one arrive.expect_tx per producer warp
+        mbar_init(&b[i], kSGroupWarps);  // full: one arrive.expect_tx per warp of the group
         mbar_init(&b[S + i], 1);   // empty: the MMA commit
       }
       mbar_init(&b[2 * S + 0], 1);    // acc_full[0]
@@ -1078,15 +1101,29 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
     tmem_alloc(tmem_slot, kSTmemCols);
     tmem_relinquish();
   }
+  // The strand's tiles, two ahead of the one entered: the id of the tile after
+  // next is loaded when a tile is entered, and the mask words of the next one,
+  // so that neither load is waited for at a tile's start (that took ~3,000
+  // cycles of every group, and ~1,500 of the MMA warp, per tile).
+  const int nstr = static_cast<int>(gridDim.x) * kStrands;
+  const int strand = warp < kEpiWarps ? 0 : (warp - kEpiWarps) / (kSProd + 1);
+  // consecutive positions sit on consecutive CTAs (so on different SMs)
+  const int pos = strand * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x);
+  int t_cur = -1, t_next = -1;
+  uint32_t w[4] = {0u, 0u, 0u, 0u};
+  if (warp >= kEpiWarps) {
+    t_cur = strand_tile(P, pos, nstr, 0);
+    t_next = strand_tile(P, pos, nstr, 1);
+    if (t_cur >= 0) load_mask_words(A, t_cur / A.n_tiles, lane, w);
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const int64_t nstr = static_cast<int64_t>(gridDim.x) * kStrands;
 
   if (warp >= kEpiWarps) {
     const int sw = warp - kEpiWarps;
-    const int s = sw / (kSProd + 1);
+    const int s = strand;
     const int role = sw % (kSProd + 1);  // < kSProd: producer warp, kSProd: MMA warp
     uint64_t *full = bars + s * kSBars;
     uint64_t *empty = full + S;
@@ -1094,127 +1131,86 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
     uint64_t *acc_empty = acc_full + 2;
     uint64_t *tile_bar = acc_full + 4;
     uint64_t *drain_bar = acc_full + 6;
-    // this strand's position in the schedule: consecutive positions sit on
-    // consecutive CTAs (so on different SMs)
-    const int64_t pos = static_cast<int64_t>(s) * gridDim.x + blockIdx.x;
     const uint32_t ring = smem_base + static_cast<uint32_t>(s * S) * P.stage_bytes;
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
-    {
-      const int64_t t0 = strand_tile(P, pos, nstr, 0);
-      if (t0 >= 0) load_mask_words(A, t0 / A.n_tiles, lane, w);
-    }
     if (role < kSProd) {
       // ---------------------------------------------------------------- producers
-      // Warp pw gathers rows [32 pw, 32 pw + 32) of every chunk: lanes 0-7
-      // each take the four sorted indices of their rows for the chunk's
-      // offset (gated by the row group's sub-tile mask; rows past M read as
-      // -1) and issue one tile::gather4.  The warp whose turn it is adds the
-      // weight slab.  A cursor runs two chunks ahead of the chunk being
-      // issued and loads their indices, so an index load's latency overlaps
-      // the two chunks before it.
-      const int pw = role;
+      // Groups of two warps take the strand's chunks in turn; a warp gathers
+      // 64 rows of its group's chunk, lanes 0-15 one tile::gather4 each (four
+      // sorted indices of the chunk's offset, gated by the row group's sub-tile
+      // mask; rows past M read as -1).  A gather4 takes about 130 cycles of a
+      // warp's issue and a chunk about 700 cycles of waits and set-up, so the
+      // strand's rate is the chunks in flight over their sum.  The group's
+      // first warp adds the weight slab.  A cursor runs one of the group's
+      // chunks ahead of the one being issued and loads its indices.
+      const int grp = role / kSGroupWarps;
+      const int half = role - grp * kSGroupWarps;
       const int esz = kF8 ? 1 : 2;
       const int box = rb / esz;
-      const uint32_t a_tx = 32u * static_cast<uint32_t>(rb);
+      constexpr int kRows = kTileM / kSGroupWarps;
+      constexpr uint32_t a_tx = kRows * rb;
       const uint32_t b_tx = static_cast<uint32_t>(A.BN) * static_cast<uint32_t>(rb);
-      const int r0 = pw * 32 + lane * 4;
-      // cursor (warp-uniform): tile (the strand's c_it-th), offsets not
-      // started yet, current offset / column block
-      int64_t c_it = -1, c_tile = -1, c_tile_m = 0;
+      const int r0 = half * kRows + lane * 4;  // lanes < kRows / 4
+      // cursor (warp-uniform but for c_sub): offsets of the tile not started yet, current offset / column block
+      int c_it = 0, c_row = 0;  // c_it: tiles entered
       uint32_t c_mm = 0u, c_sub = 0u;
-      int c_k = 0, c_cb = 0, c_n0 = 0;
-      bool c_valid = true;
-      // enters the following tiles until one visits an offset (writing
-      // mask_output for each tile entered)
-      auto next_tile = [&]() {
-        for (;;) {
-          c_tile = strand_tile(P, pos, nstr, ++c_it);
-          if (c_tile < 0) {
-            c_valid = false;
-            return;
-          }
-          const TileMasks t = reduce_masks(A, w);
-          const int64_t t_next = strand_tile(P, pos, nstr, c_it + 1);
-          if (t_next >= 0) load_mask_words(A, t_next / A.n_tiles, lane, w);
-          c_tile_m = c_tile / A.n_tiles;
-          const int n_tile = static_cast<int>(c_tile % A.n_tiles);
-          c_n0 = n_tile * A.BN;
-          if (pw == 0 && lane == 0 && A.is_fwd && A.mask_out != nullptr && n_tile == 0) {
-            const int nsub = kTileM / A.tile_m_desp;
-            for (int d = 0; d < nsub; ++d) {
-              const int64_t start = c_tile_m * kTileM + d * A.tile_m_desp;
-              if (start >= A.M) break;
-              uint32_t wd;
-              if (nsub == 4) wd = t.g[d];
-              else if (nsub == 2) wd = d == 0 ? (t.g[0] | t.g[1]) : (t.g[2] | t.g[3]);
-              else wd = t.g[0] | t.g[1] | t.g[2] | t.g[3];
-              A.mask_out[start / A.tile_m_desp] = wd & A.mask_filter;
-            }
-          }
-          // rows of lanes 0-7 lie in 32-row group pw
-          c_sub = pw == 0 ? t.sub[0] : pw == 1 ? t.sub[1] : pw == 2 ? t.sub[2] : t.sub[3];
-          if (t.tm != 0u) {
-            c_k = __ffs(t.tm) - 1;
-            c_mm = t.tm & (t.tm - 1u);
+      int c_k = 0, c_cb = P.cpo - 1, c_nt = 0;
+      // the group's chunk to issue: this lane's indices, and offset | column
+      // block << 5 | column tile << 16 (-1: none)
+      int4 q0 = make_int4(-1, -1, -1, -1);
+      int d0 = -1;
+      uint32_t stage = static_cast<uint32_t>(grp), eph = 0, gchunk = 0;
+      for (bool first = true;; first = false) {
+        // the group's next chunk: the strand's next kSGroups (first: grp + 1)
+        for (int skip = first ? grp : kSGroups - 1; skip >= 0 && c_k >= 0; --skip) {
+          if (++c_cb >= P.cpo) {
             c_cb = 0;
-            return;
+            // enter the following tiles until one visits an offset (writing
+            // mask_output for each tile entered)
+            while (c_mm == 0u) {
+              const int c_tile = t_cur;
+              if (c_tile < 0) break;
+              const TileMasks t = reduce_masks(A, w);
+              t_cur = t_next;
+              if (t_cur >= 0) load_mask_words(A, t_cur / A.n_tiles, lane, w);
+              t_next = strand_tile(P, pos, nstr, ++c_it + 1);
+              const int c_tile_m = c_tile / A.n_tiles;
+              c_nt = c_tile - c_tile_m * A.n_tiles;
+              c_row = c_tile_m * kTileM + r0;
+              if (role == 0 && lane == 0 && A.is_fwd && A.mask_out != nullptr && c_nt == 0) {
+                const int nsub = kTileM / A.tile_m_desp;
+                for (int d = 0; d < nsub; ++d) {
+                  const int start = c_tile_m * kTileM + d * A.tile_m_desp;
+                  if (start >= A.M) break;
+                  uint32_t wd;
+                  if (nsub == 4) wd = d == 0 ? t.g[0] : d == 1 ? t.g[1] : d == 2 ? t.g[2] : t.g[3];
+                  else if (nsub == 2) wd = d == 0 ? (t.g[0] | t.g[1]) : (t.g[2] | t.g[3]);
+                  else wd = t.g[0] | t.g[1] | t.g[2] | t.g[3];
+                  A.mask_out[start / A.tile_m_desp] = wd & A.mask_filter;
+                }
+              }
+              // this lane's rows lie in 32-row group r0 / 32
+              const int q = r0 >> 5;
+              c_sub = q == 0 ? t.sub[0] : q == 1 ? t.sub[1] : q == 2 ? t.sub[2] : t.sub[3];
+              c_mm = t.tm;
+            }
+            c_k = __ffs(c_mm) - 1;  // -1: past the strand's last tile
+            c_mm &= c_mm - 1u;
           }
         }
-      };
-      auto advance = [&]() {
-        if (++c_cb < P.cpo) return;
-        c_cb = 0;
-        if (c_mm != 0u) {
-          c_k = __ffs(c_mm) - 1;
-          c_mm &= c_mm - 1u;
-          return;
-        }
-        next_tile();
-      };
-      // this lane's four indices of the cursor's chunk (checked when issued,
-      // so the load stays in flight until then)
-      auto load_q = [&]() {
-        int4 q = make_int4(-1, -1, -1, -1);
-        const int64_t rg = c_tile_m * kTileM + r0;
-        if (lane < 8 && rg < A.M && ((c_sub >> c_k) & 1u))
-          q = __ldg(reinterpret_cast<const int4 *>(A.idx_sorted + static_cast<int64_t>(c_k) * A.M + rg));
-        return q;
-      };
-      next_tile();
-      // slots 0 (the chunk to issue) and 1 (the next one)
-      int4 q0 = make_int4(-1, -1, -1, -1), q1 = q0;
-      int k0 = 0, cb0 = 0, n00 = 0, k1 = 0, cb1 = 0, n01 = 0;
-      bool v0 = c_valid, v1 = false;
-      if (c_valid) {
-        q0 = load_q();
-        k0 = c_k; cb0 = c_cb; n00 = c_n0;
-        advance();
-        v1 = c_valid;
-        if (c_valid) {
-          q1 = load_q();
-          k1 = c_k; cb1 = c_cb; n01 = c_n0;
-          advance();
-        }
-      }
-      uint32_t stage = 0, eph = 0, gchunk = 0;
-      while (v0) {
-        // the chunk two ahead: load its indices now
-        int4 q2 = make_int4(-1, -1, -1, -1);
-        int k2 = 0, cb2 = 0, n02 = 0;
-        const bool v2 = c_valid;
-        if (v2) {
-          q2 = load_q();
-          k2 = c_k; cb2 = c_cb; n02 = c_n0;
-          advance();
-        }
-        if (!__all_sync(0xffffffffu, mbar_wait(&empty[stage], eph ^ 1u, abort_flag))) {
-          if (lane == 0) flag_error(A.err, kErrWaitTimeout);
-          break;
-        }
-        const uint32_t sA = ring + stage * P.stage_bytes;
-        if (lane == 0) {
-          if (static_cast<int>(gchunk % kSProd) == pw) {
-            mbar_arrive_expect_tx(&full[stage], a_tx + b_tx);
+        int4 q1 = make_int4(-1, -1, -1, -1);
+        if (c_k >= 0 && lane < kRows / 4 && c_row < static_cast<int>(A.M) && ((c_sub >> c_k) & 1u))
+          q1 = __ldg(reinterpret_cast<const int4 *>(A.idx_sorted + static_cast<int64_t>(c_k) * A.M + c_row));
+        if (d0 >= 0) {
+          if (!__all_sync(0xffffffffu, mbar_wait(&empty[stage], eph ^ 1u, abort_flag))) {
+            if (lane == 0) flag_error(A.err, kErrWaitTimeout);
+            break;
+          }
+          const uint32_t sA = ring + stage * P.stage_bytes;
+          const int cb0 = (d0 >> 5) & 2047;
+          if (lane == 0) mbar_arrive_expect_tx(&full[stage], half == 0 ? a_tx + b_tx : a_tx);
+          __syncwarp();
+          if (half == 0 && elect_one()) {
+            const int k0 = d0 & 31, n00 = (d0 >> 16) * A.BN;
             if (P.b_mn) {
               for (int qq = 0; qq < A.BN / 64; ++qq)
                 tma_load_2d(sA + P.b_off + qq * 8192, &P.tmap_b, k0 * (A.b_off_stride / esz) + n00 + 64 * qq,
@@ -1222,31 +1218,31 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
             } else {
               tma_load_2d(sA + P.b_off, &P.tmap_b, k0 * (A.b_off_stride / esz) + cb0 * box, n00, &full[stage]);
             }
-          } else {
-            mbar_arrive_expect_tx(&full[stage], a_tx);
           }
-        }
-        __syncwarp();
-        if (lane < 8) {
-          if (q0.x < -1 || q0.x >= A.a_rows || q0.y < -1 || q0.y >= A.a_rows || q0.z < -1 || q0.z >= A.a_rows ||
-              q0.w < -1 || q0.w >= A.a_rows) {
-            flag_error(A.err, kErrBadIndex);
-            q0 = make_int4(-1, -1, -1, -1);
+          if (lane < kRows / 4) {
+            const int n = static_cast<int>(A.a_rows);
+            if (q0.x < -1 || q0.x >= n || q0.y < -1 || q0.y >= n || q0.z < -1 || q0.z >= n || q0.w < -1 || q0.w >= n) {
+              flag_error(A.err, kErrBadIndex);
+              q0 = make_int4(-1, -1, -1, -1);
+            }
+            if (P.zero_ok && (q0.x & q0.y & q0.z & q0.w) == -1) {
+              const int z = zero_group(blockIdx.x * 128 + role * 16 + lane, gchunk);
+              tma_gather4(sA + r0 * rb, &P.tmap_zero, 0, z, z + 1, z + 2, z + 3, &full[stage]);
+            } else {
+              tma_gather4(sA + r0 * rb, &P.tmap_a, cb0 * box, q0.x, q0.y, q0.z, q0.w, &full[stage]);
+            }
           }
-          if (P.zero_ok && (q0.x & q0.y & q0.z & q0.w) == -1) {
-            const int z = zero_group(blockIdx.x * 64 + warp * 8 + lane, gchunk);
-            tma_gather4(sA + r0 * rb, &P.tmap_zero, 0, z, z + 1, z + 2, z + 3, &full[stage]);
+          ++gchunk;
+          stage += kSGroups;
+          if (stage >= static_cast<uint32_t>(S)) {
+            stage -= static_cast<uint32_t>(S);
+            eph ^= 1u;
           }
-          else
-            tma_gather4(sA + r0 * rb, &P.tmap_a, cb0 * box, q0.x, q0.y, q0.z, q0.w, &full[stage]);
+        } else if (!first) {
+          break;
         }
-        ++gchunk;
-        if (++stage == static_cast<uint32_t>(S)) {
-          stage = 0;
-          eph ^= 1u;
-        }
-        q0 = q1; k0 = k1; cb0 = cb1; n00 = n01; v0 = v1;
-        q1 = q2; k1 = k2; cb1 = cb2; n01 = n02; v1 = v2;
+        q0 = q1;
+        d0 = c_k < 0 ? -1 : c_k | c_cb << 5 | c_nt << 16;
       }
     } else {
       // ---------------------------------------------------------------- MMA warp
@@ -1259,14 +1255,14 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
       uint32_t stage = 0, fph = 0;
       bool issued = false, ok = true;
       for (int it = 0;; ++it) {
-        const int64_t tile = strand_tile(P, pos, nstr, it);
+        const int tile = t_cur;
         const bool have = tile >= 0;
         int nch = 0;
         if (have) {
-          const TileMasks tmk = reduce_masks(A, w);
-          const int64_t t_next = strand_tile(P, pos, nstr, it + 1);
-          if (t_next >= 0) load_mask_words(A, t_next / A.n_tiles, lane, w);
-          nch = __popc(tmk.tm) * P.cpo;
+          nch = __popc(reduce_masks(A, w).tm) * P.cpo;
+          t_cur = t_next;
+          if (t_cur >= 0) load_mask_words(A, t_cur / A.n_tiles, lane, w);
+          t_next = strand_tile(P, pos, nstr, it + 2);
         }
         if (elect_one()) {
           const int ab = it & 1;
@@ -1330,22 +1326,18 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
     // Takes the strands' accumulators in turn; thread r owns TMEM lane r (tile row r).
     const int r = threadIdx.x;
     const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    int its[kStrands];
-    bool done[kStrands];
-    for (int s = 0; s < kStrands; ++s) {
-      its[s] = 0;
-      done[s] = false;
-    }
-    int n_done = 0;
+    // per strand: two bits of its tile count (buffer, phase); bits 8+: finished
+    uint32_t turn = 0u;
     bool ok = true;
-    while (n_done < kStrands && ok) {
+    while ((turn >> 8) != (1u << kStrands) - 1u && ok) {
       for (int s = 0; s < kStrands && ok; ++s) {
-        if (done[s]) continue;
+        if ((turn >> (8 + s)) & 1u) continue;
         uint64_t *acc_full = bars + s * kSBars + 2 * S;
         uint64_t *acc_empty = acc_full + 2;
         uint64_t *tile_bar = acc_full + 4;
-        const int ab = its[s] & 1;
-        const uint32_t aph = (its[s] >> 1) & 1;
+        const uint32_t its = (turn >> (2 * s)) & 3u;
+        const int ab = static_cast<int>(its & 1u);
+        const uint32_t aph = its >> 1;
         if (!mbar_wait(&tile_bar[ab], aph, abort_flag)) {
           flag_error(A.err, kErrWaitTimeout);
           ok = false;
@@ -1353,8 +1345,7 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
         }
         const int tile = acc_tile[s * 2 + ab];
         if (tile < 0) {
-          done[s] = true;
-          ++n_done;
+          turn |= 1u << (8 + s);
           continue;
         }
         const int64_t tile_m = tile / A.n_tiles;
@@ -1369,8 +1360,7 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
           const int64_t rr = tile_m * kTileM + q * 32 + lane;
           if (rr < A.M) km |= A.mask ? __ldg(A.mask + rr) : 1u;
         }
-#pragma unroll
-        for (int sh = 16; sh > 0; sh >>= 1) km |= __shfl_xor_sync(0xffffffffu, km, sh);
+        km = __reduce_or_sync(0xffffffffu, km);
         km &= A.mask_filter;
         if (!mbar_wait(&acc_full[ab], aph, abort_flag)) {
           flag_error(A.err, kErrWaitTimeout);
@@ -1392,7 +1382,7 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
         }
         tc_fence_before();
         mbar_arrive(&acc_empty[ab]);
-        ++its[s];
+        turn = (turn & ~(3u << (2 * s))) | (((its + 1u) & 3u) << (2 * s));
       }
     }
   }
@@ -1466,7 +1456,8 @@ cudaError_t launch_conv_rowgather(const ConvRowGatherArgs &a, int num_sms, cudaS
   P.row_bytes = 128;
   P.bulk_idx = a.idx_sorted != nullptr && reinterpret_cast<uintptr_t>(a.idx_sorted) % 16 == 0 &&
                a.M % 4 == 0;
-  if (a.a_row_bytes == 64 && a.kv > 1 && a.a_rows > 0 &&
+  const bool rows16 = a.a_rows > 0 && reinterpret_cast<uintptr_t>(a.a_base) % 16 == 0 && a.a_row_stride % 16 == 0;
+  if (a.a_row_bytes == 64 && a.kv > 1 && rows16 &&
       encode_tmap_2d(&P.tmap_b, a.in_dtype, a.b_base, red * a.kv, a.n_total,
                      static_cast<uint64_t>(a.b_row_stride), 64u / esz, a.BN, 64) &&
       encode_tmap_2d(&P.tmap_a, a.in_dtype, a.a_base, red, static_cast<uint64_t>(a.a_rows),
@@ -1495,10 +1486,9 @@ cudaError_t launch_conv_rowgather(const ConvRowGatherArgs &a, int num_sms, cudaS
                                   static_cast<uint64_t>(a.b_row_stride), 64, 64)
                  : encode_tmap_2d(&P.tmap_b, a.in_dtype, a.b_base, red * a.kv, a.n_total,
                                   static_cast<uint64_t>(a.b_row_stride), box, a.BN);
-    // gathered A rows: [a_rows, red] with one-row boxes (tile::gather4)
-    if (tma && a.a_row_bytes >= 128 && a.a_rows > 0)
-      gather = encode_tmap_2d(&P.tmap_a, a.in_dtype, a.a_base, red, static_cast<uint64_t>(a.a_rows),
-                              static_cast<uint64_t>(a.a_row_stride), box, 1);
+    gather = tma && a.a_row_bytes >= 128 && rows16 &&
+             encode_tmap_2d(&P.tmap_a, a.in_dtype, a.a_base, red, static_cast<uint64_t>(a.a_rows),
+                            static_cast<uint64_t>(a.a_row_stride), box, 1);
   }
   // zero rows with the same box and swizzle as the gathered rows
   P.zero_ok = 0;
@@ -1515,14 +1505,17 @@ cudaError_t launch_conv_rowgather(const ConvRowGatherArgs &a, int num_sms, cudaS
   const uint32_t b_bytes = static_cast<uint32_t>(a.BN) * P.row_bytes;
   P.stage_bytes = a_bytes + b_bytes;
   P.b_off = a_bytes;
-  // Strands (two independent pipelines per CTA, two CTAs per SM) on the TMA
+  // Strands (one pipeline per CTA, two CTAs per SM) on the TMA
   // gather path of 128-byte rows with the sorted index table and BN <= 64
-  // (TMEM: 2 strands x 2 buffers x BN columns per CTA).
-  if (gather && P.bulk_idx && a.BN <= 64 && !(P.row_bytes == 64 && a.b_mn)) {
+  // (TMEM: 2 buffers x BN columns per CTA); the chunk word of its cursor packs
+  // the offset, 11 bits of column block and 15 of column tile, and its tile and
+  // row numbers are 32-bit.
+  if (gather && P.bulk_idx && a.BN <= 64 && !(P.row_bytes == 64 && a.b_mn) && P.cpo < 2048 && a.n_tiles < 32768 &&
+      P.num_tiles < (int64_t(1) << 30) && a.a_rows < (int64_t(1) << 31) && a.M < (int64_t(1) << 31) - 1024) {
     if (P.num_tiles == 0) return cudaSuccess;
-    // two CTAs per SM (113 KB each): two stages per strand with 128-byte rows
-    // (24 KB at BN 64), four with 64-byte rows (12 KB)
-    const int stages = P.row_bytes == 128 ? 2 : 4;
+    // two CTAs per SM (113 KB each): four stages with 128-byte rows (24 KB at
+    // BN 64), eight with 64-byte rows (12 KB)
+    const int stages = P.row_bytes == 128 ? 4 : 8;
     P.stages = stages;
     P.tmem_cols = kSTmemCols;
     P.bar_off = P.stage_bytes * kStrands * stages;
@@ -1569,6 +1562,9 @@ cudaError_t launch_conv_rowgather(const ConvRowGatherArgs &a, int num_sms, cudaS
   const int stages = stages_for(pair ? kLimitPair : kLimitSingle, idx_stages);
   if (stages < 2) return cudaErrorInvalidConfiguration;
   P.stages = stages;
+  // one warp per chunk where the ring has a stage for every warp, else two, else four
+  const int prod = pair ? Layout<true>::kProdWarps : Layout<false>::kProdWarps;
+  P.group_warps = stages >= prod ? 1 : stages >= prod / 2 ? 2 : 4;
   P.idx_off = P.stage_bytes * stages;
   P.bar_off = P.idx_off + P.idx_buf_bytes * idx_stages;
   const size_t smem = 1024 + P.bar_off + bar_bytes;
