@@ -84,6 +84,7 @@ struct WParams {
   int n_mma;           // MMA N (K rounded up to 64)
   int mw_shift;        // log2(mask_width) when it is a power of two, else -1
   int stages;
+  int group_warps;     // gather path, single layout: producer warps per stage
   uint32_t stage_bytes;
   uint32_t b_off;
   uint32_t bbuf_off;      // gather path: n_bbuf dOut buffers of n_b_atoms x 8 KB
@@ -211,9 +212,9 @@ __global__ void __maxnreg__(kPair ? 80 : 96) conv_wgrad_kernel(const __grid_cons
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S; ++i) {
-      // gather: one arrive.expect_tx per producer warp; cp.async: the 32
+      // gather: one arrive.expect_tx per warp of the group; cp.async: the 32
       // lanes of the stage's producer warp (cp.async.mbarrier.arrive.noinc)
-      mbar_init(&full_bar[i], kGather ? kProdWarps : 32);
+      mbar_init(&full_bar[i], kGather ? (kPair ? kProdWarps : P.group_warps) : 32);
       mbar_init(&empty_bar[i], 1);
     }
     for (int i = 0; i < kIdxStages; ++i) {
@@ -223,7 +224,7 @@ __global__ void __maxnreg__(kPair ? 80 : 96) conv_wgrad_kernel(const __grid_cons
     mbar_init(acc_full, 1);
     mbar_init(drain_bar, 1);
     for (int i = 0; i < kMaxBBufs; ++i) {
-      mbar_init(&bfull[i], kProdWarps);
+      mbar_init(&bfull[i], kPair ? kProdWarps : P.group_warps);
       mbar_init(&bempty[i], 1);
     }
     *abort_flag = 0;
@@ -241,25 +242,34 @@ __global__ void __maxnreg__(kPair ? 80 : 96) conv_wgrad_kernel(const __grid_cons
   const uint32_t tmem_base = *tmem_slot;
 
   // ---------------------------------------------------------------- TMA gather producer loop
-  // Producer warps of ring `ring` serve every stage of that ring: warp pw
-  // owns rows [kRpw pw, kRpw pw + kRpw) of each 64-row atom; lane l < 2 kGpw
-  // issues one tile::gather4 for rows kRpw pw + 4 (l % kGpw) .. +3 of atom
-  // l / kGpw (input rows of the atom's filter; a group of four absent rows
-  // reads the zero tensor).  The chunk's 64 dOut rows are the same for every
-  // M-tile, so they are gathered once per chunk into one of the ring's dOut
-  // buffers (lanes l < kGpw n_b_atoms, same row split), released by the MMA
-  // after the chunk's last tile.  Lane 0 of each warp arrives with
-  // expect_tx for its bytes.  With two rings (pair layout) ring r takes the
-  // CTA's chunks it = r, r + 2, ... (index buffers it % 4: 0 and 2 for ring
-  // 0, 1 and 3 for ring 1), and owns half of the stages and dOut buffers.
+  // The producer warps of ring `ring` form groups of P.group_warps that take the
+  // ring's stages (and, apart from those, its chunks' dOut rows) in turn: a
+  // stage costs a warp ~500 cycles of waits and set-up beside ~110 per
+  // gather4.  Warp wi of a group owns rows [kRpw wi, kRpw wi + kRpw) of each
+  // 64-row atom; lane l < 2 kGpw issues one tile::gather4 for rows kRpw wi +
+  // 4 (l % kGpw) .. +3 of atom l / kGpw (input rows of the atom's filter; a
+  // group of four absent rows reads the zero tensor).  The chunk's 64 dOut rows
+  // are the same for every M-tile, so they are gathered once per chunk into one
+  // of the ring's dOut buffers (lanes l < kGpw n_b_atoms, same row split),
+  // released by the MMA after the chunk's last tile.  Lane 0 of each warp of
+  // the group arrives with expect_tx for its bytes.  The groups are at most as
+  // many as the ring's stages and buffers: the parity of a stage that a group
+  // tests is then never two uses behind.  With two rings (pair layout) ring r
+  // takes the CTA's chunks it = r, r + 2, ... (index buffers it % 4: 0 and 2
+  // for ring 0, 1 and 3 for ring 1), owns half of the stages and dOut buffers,
+  // and is one group: its two stages would be held longer than groups save.
   auto produce_gather = [&](int pw, int ring) {
-    constexpr int kRpw = kRows / kProdWarps;  // rows per warp: 8 single, 16 pair
-    constexpr int kGpw = kRpw / 4;            // gathers per atom per warp
+    const int W = kPair ? kProdWarps : P.group_warps;
+    const int groups = kProdWarps / W;
+    const int kRpw = kRows / W;               // rows per warp
+    const int kGpw = kRpw / 4;                // gathers per atom per warp
+    const int grp = pw / W, wi = pw - grp * W;
     const int n_b_atoms = P.n_mma / 64;
     const uint32_t Sr = static_cast<uint32_t>(S / kRings);
     const uint32_t NBr = P.n_bbuf / kRings;
-    const int rq = pw * kRpw + (lane % kGpw) * 4;
+    const int rq = wi * kRpw + (lane % kGpw) * 4;
     uint32_t stage = 0, eph = 0, bb = 0, bph = 0;  // this ring's stage / dOut buffer and phases
+    int turn = 0, bturn = 0;                       // stage / used chunk % groups
     bool ok = true;
     int it = ring;
     for (int c = c_begin + ring * c_step; c < c_end && ok; c += kRings * c_step, it += kRings) {
@@ -275,24 +285,27 @@ __global__ void __maxnreg__(kPair ? 80 : 96) conv_wgrad_kernel(const __grid_cons
       const WMeta *meta = reinterpret_cast<const WMeta *>(sig_tab + kRows);
       uint32_t bits = meta->active_bits;
       if (bits) {
-        const uint32_t bi = static_cast<uint32_t>(ring) * NBr + bb;
-        if (!__all_sync(0xffffffffu, mbar_wait(&bempty[bi], bph ^ 1u, abort_flag))) {
-          if (lane == 0) flag_error(A.err, kErrWaitTimeout);
-          break;
-        }
-        if (lane == 0) mbar_arrive_expect_tx(&bfull[bi], static_cast<uint32_t>(n_b_atoms * kRpw) * 128u);
-        __syncwarp();
-        if (lane < kGpw * n_b_atoms) {
-          const int na = lane / kGpw;
-          const int4 q = *reinterpret_cast<const int4 *>(sig_tab + rq);
-          const uint32_t dst = smem_base + P.bbuf_off + bi * (n_b_atoms * 8192u) + na * 8192u + rq * 128;
-          if (P.zero_ok && (q.x & q.y & q.z & q.w) == -1) {
-            const int z = zero_group(blockIdx.x * 64 + pw * 8 + lane, static_cast<uint32_t>(it));
-            tma_gather4(dst, &P.tmap_zero, 0, z, z + 1, z + 2, z + 3, &bfull[bi]);
+        if (bturn == grp) {
+          const uint32_t bi = static_cast<uint32_t>(ring) * NBr + bb;
+          if (!__all_sync(0xffffffffu, mbar_wait(&bempty[bi], bph ^ 1u, abort_flag))) {
+            if (lane == 0) flag_error(A.err, kErrWaitTimeout);
+            break;
           }
-          else
-            tma_gather4(dst, &P.tmap_dout, na * 64, q.x, q.y, q.z, q.w, &bfull[bi]);
+          if (lane == 0) mbar_arrive_expect_tx(&bfull[bi], static_cast<uint32_t>(n_b_atoms * kRpw) * 128u);
+          __syncwarp();
+          for (int l = lane; l < kGpw * n_b_atoms; l += 32) {
+            const int na = l / kGpw;
+            const int4 q = *reinterpret_cast<const int4 *>(sig_tab + rq);
+            const uint32_t dst = smem_base + P.bbuf_off + bi * (n_b_atoms * 8192u) + na * 8192u + rq * 128;
+            if (P.zero_ok && (q.x & q.y & q.z & q.w) == -1) {
+              const int z = zero_group(blockIdx.x * 64 + pw * 8 + lane, static_cast<uint32_t>(it));
+              tma_gather4(dst, &P.tmap_zero, 0, z, z + 1, z + 2, z + 3, &bfull[bi]);
+            } else {
+              tma_gather4(dst, &P.tmap_dout, na * 64, q.x, q.y, q.z, q.w, &bfull[bi]);
+            }
+          }
         }
+        if (++bturn == groups) bturn = 0;
         if (++bb == NBr) {
           bb = 0;
           bph ^= 1u;
@@ -301,32 +314,35 @@ __global__ void __maxnreg__(kPair ? 80 : 96) conv_wgrad_kernel(const __grid_cons
       while (bits) {
         const int jt = __ffs(bits) - 1;
         bits &= bits - 1;
-        const int tt = t0 + jt;
-        const uint32_t s = static_cast<uint32_t>(ring) * Sr + stage;
-        if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], eph ^ 1, abort_flag))) {
-          if (lane == 0) flag_error(A.err, kErrWaitTimeout);
-          ok = false;
-          break;
+        if (turn == grp) {
+          const int tt = t0 + jt;
+          const uint32_t s = static_cast<uint32_t>(ring) * Sr + stage;
+          if (!__all_sync(0xffffffffu, mbar_wait(&empty_bar[s], eph ^ 1, abort_flag))) {
+            if (lane == 0) flag_error(A.err, kErrWaitTimeout);
+            ok = false;
+            break;
+          }
+          if (lane == 0) mbar_arrive_expect_tx(&full_bar[s], 2u * kRpw * 128u);
+          __syncwarp();
+          if (lane < 2 * kGpw) {
+            const int a = 2 * tt + lane / kGpw;
+            const int k = a / P.cpa;
+            int4 q = make_int4(-1, -1, -1, -1);
+            if (a < P.n_atoms && k < A.kv)
+              q = *reinterpret_cast<const int4 *>(tab + (k - k_lo) * kRows + rq);
+            const uint32_t dst = smem_base + s * P.stage_bytes + (lane / kGpw) * 8192u + rq * 128;
+            if (P.zero_ok && (q.x & q.y & q.z & q.w) == -1) {
+              const int z = zero_group(blockIdx.x * 64 + pw * 8 + lane, s + static_cast<uint32_t>(it));
+              tma_gather4(dst, &P.tmap_zero, 0, z, z + 1, z + 2, z + 3, &full_bar[s]);
+            } else {
+              tma_gather4(dst, &P.tmap_in, (a % P.cpa) * 64, q.x, q.y, q.z, q.w, &full_bar[s]);
+            }
+          }
         }
+        if (++turn == groups) turn = 0;
         if (++stage == Sr) {
           stage = 0;
           eph ^= 1u;
-        }
-        if (lane == 0) mbar_arrive_expect_tx(&full_bar[s], 2u * kRpw * 128u);
-        __syncwarp();
-        if (lane < 2 * kGpw) {
-          const int a = 2 * tt + lane / kGpw;
-          const int k = a / P.cpa;
-          int4 q = make_int4(-1, -1, -1, -1);
-          if (a < P.n_atoms && k < A.kv)
-            q = *reinterpret_cast<const int4 *>(tab + (k - k_lo) * kRows + rq);
-          const uint32_t dst = smem_base + s * P.stage_bytes + (lane / kGpw) * 8192u + rq * 128;
-          if (P.zero_ok && (q.x & q.y & q.z & q.w) == -1) {
-            const int z = zero_group(blockIdx.x * 64 + pw * 8 + lane, s + static_cast<uint32_t>(it));
-            tma_gather4(dst, &P.tmap_zero, 0, z, z + 1, z + 2, z + 3, &full_bar[s]);
-          }
-          else
-            tma_gather4(dst, &P.tmap_in, (a % P.cpa) * 64, q.x, q.y, q.z, q.w, &full_bar[s]);
         }
       }
       if (!ok) break;
@@ -925,14 +941,16 @@ cudaError_t launch_conv_wgrad(const ConvWgradArgs &a, int num_sms, cudaStream_t 
   per_group = (P.n_mtiles + n_groups - 1) / n_groups;
   P.tiles_per_group = per_group;
   P.n_groups = (P.n_mtiles + per_group - 1) / per_group;
-  // row splits: the caller's split_k_slices, else about one CTA per SM (two
-  // per SM in the pair layout)
+  // row splits: the caller's split_k_slices, else as many CTAs as run at once
+  // (one per SM, two in the pair layout): rounding the splits up left a second
+  // wave of a few CTAs (60k voxels, C = K = 128: 7 groups x 22 splits on 148 SMs)
   const int ctas = (pair ? 2 : 1) * num_sms;
-  int splits = a.split_k > 0 ? a.split_k : (ctas + P.n_groups - 1) / P.n_groups;
+  int splits = a.split_k > 0 ? a.split_k : ctas > P.n_groups ? ctas / P.n_groups : 1;
   if (splits > P.n_chunks) splits = P.n_chunks;
   P.chunks_per_cta = (P.n_chunks + splits - 1) / splits;
   splits = (P.n_chunks + P.chunks_per_cta - 1) / P.chunks_per_cta;
   P.stages = stages;
+  P.group_warps = stages >= 4 && P.n_bbuf >= 4 ? 2 : 4;
   P.bbuf_off = P.stage_bytes * stages;
   P.idx_off = P.bbuf_off + bbuf_bytes;
   P.bar_off = P.idx_off + P.idx_buf_bytes * kIdxStages;
