@@ -70,6 +70,8 @@ def lib_path() -> Path:
 def load() -> ctypes.CDLL:
     """Loads the library (once).  Raises RuntimeError if it is missing."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
@@ -126,7 +128,22 @@ def device_error_bits(stream: int = 0) -> int:
     return int(bits.value)
 
 
+_have_cuda = False
+
+
 def require_cuda():
+    """Raises RuntimeError without a CUDA device (asked until there is one)."""
+    global _have_cuda
+    if _have_cuda:
+        return
     import torch
     if not torch.cuda.is_available():
         raise RuntimeError("cumm B200 kernels need a CUDA device (there is no CPU fallback)")
+    _have_cuda = True
+
+
+def current_stream() -> int:
+    """cudaStream_t of the current device's current torch stream (the value of
+    torch.cuda.current_stream().cuda_stream, without building its objects)."""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())

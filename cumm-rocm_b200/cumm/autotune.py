@@ -11,11 +11,13 @@ The reference picks its kernel from a fixed if-tree over tile shapes
 (cumm/conv/main.py:483-745, 'Can't Found Algorithm' when none fits); here the
 candidates all compute the same result and only their speed differs.
 """
+import functools
 from dataclasses import dataclass, field
 from typing import Callable, Dict, List, Sequence, Tuple
 
 import torch
 
+from cumm import _lib
 from cumm import tensorview as tv
 from cumm.conv.main import ConvMainUnitTest, get_all_conv_algo_desp
 from cumm.tensorview.gemm import ConvOpType, ConvParams
@@ -50,6 +52,7 @@ def fwd_candidates(K: int) -> List[FwdConfig]:
     return res
 
 
+@functools.lru_cache(maxsize=None)
 def _desp(dt_in, dt_out):
     for d in get_all_conv_algo_desp():
         if (d.op_type == ConvOpType.kForward and d.algo == "Tcgen05" and d.dtype_input == dt_in
@@ -83,7 +86,7 @@ def run_forward(cfg: FwdConfig, x: torch.Tensor, w: torch.Tensor, out: torch.Ten
             p.scale = tv.Tensor(scale)
         if act_type and j == cfg.num_split - 1:
             p.act_type = act_type
-        p.stream = stream or torch.cuda.current_stream().cuda_stream
+        p.stream = stream or _lib.current_stream()
         cm.implicit_gemm2(p)
 
 
@@ -112,7 +115,7 @@ def run_wgrad(cfg: WgradConfig, x: torch.Tensor, dy: torch.Tensor, dw: torch.Ten
     p.indices_sorted = tv.Tensor(pt.sorted_indices("fwd"))
     p.mask_width = 128
     p.split_k_slices = cfg.split_k if cfg.split_k > 1 else 1
-    p.stream = stream or torch.cuda.current_stream().cuda_stream
+    p.stream = stream or _lib.current_stream()
     cm.implicit_gemm2(p)
 
 

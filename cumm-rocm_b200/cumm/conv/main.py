@@ -52,9 +52,6 @@ class _Workspace:
 _WS = _Workspace()
 
 
-def _ptr(t: tv.Tensor):
-    return None if t is None or t.empty() else t.byte_pointer()
-
 
 def _algo_code(desp) -> int:
     if desp.algo in SIMT_ALGOS:
@@ -64,11 +61,16 @@ def _algo_code(desp) -> int:
     raise RuntimeError(f"Can't Found Algorithm for params: {desp.algo}")
 
 
-def _check_dense(t: tv.Tensor, name: str):
-    if not t.empty() and not t.is_contiguous():
+def _dense_ptr(t: tv.Tensor, name: str):
+    """Device address of a dense CUDA tensor, None for an empty one."""
+    x = t._t
+    if x is None or x.numel() == 0:
+        return None
+    if not x.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
-    if not t.empty() and t.device < 0:
+    if x.device.type == "cpu":
         raise ValueError(f"{name} must be a CUDA tensor")
+    return x.data_ptr()
 
 
 def build_conv_params_c(params: ConvParams) -> Tuple[_lib.ConvParamsC, dict]:
@@ -83,24 +85,27 @@ def build_conv_params_c(params: ConvParams) -> Tuple[_lib.ConvParamsC, dict]:
         raise RuntimeError("error: weight must be [K, kv, C]")
     if out.ndim != 2:
         raise RuntimeError("error: output must be [N, K]")
-    K = w.dim(0)
-    kv = w.dim(1)
-    C = inp.dim(1)
-    if out.dim(1) != K:
+    K, kv, wc = w._t.shape
+    n_in, C = inp._t.shape
+    n_out, out_cols = out._t.shape
+    if out_cols != K:
         raise RuntimeError("error: output.dim(1) != weight.dim(0)")
-    if w.dim(2) != C:
+    if wc != C:
         raise RuntimeError("error: weight.dim(2) != input.dim(1)")
-    for t, n in ((inp, "input"), (w, "weight"), (out, "output"), (params.indices, "indices"),
-                 (params.mask, "mask"), (params.mask_argsort, "mask_argsort"),
-                 (params.mask_output, "mask_output"), (params.bias, "bias"),
-                 (params.scale, "scale"), (params.output_add, "output_add")):
-        _check_dense(t, n)
-    if params.indices.empty():
+    indices, mask, mask_output = params.indices, params.mask, params.mask_output
+    p_inp, p_w, p_out = _dense_ptr(inp, "input"), _dense_ptr(w, "weight"), _dense_ptr(out, "output")
+    p_indices, p_mask = _dense_ptr(indices, "indices"), _dense_ptr(mask, "mask")
+    p_argsort = _dense_ptr(params.mask_argsort, "mask_argsort")
+    p_mask_output = _dense_ptr(mask_output, "mask_output")
+    p_bias, p_scale = _dense_ptr(params.bias, "bias"), _dense_ptr(params.scale, "scale")
+    p_add = _dense_ptr(params.output_add, "output_add")
+    if p_indices is None:
         raise RuntimeError("error: indices must not be empty")
-    if params.indices.ndim != 2 or params.indices.dim(0) != kv:
-        raise RuntimeError(f"error: indices shape {params.indices.shape} != [{kv}, -1]")
-    if not params.scale.empty() and params.scale.dtype != tv.float32:
+    if indices.ndim != 2 or indices.dim(0) != kv:
+        raise RuntimeError(f"error: indices shape {indices.shape} != [{kv}, -1]")
+    if p_scale is not None and params.scale.dtype != tv.float32:
         raise ValueError("scale must be float32 [K]")
+    n_rows = indices._t.shape[1]
     op = ConvOpType(desp.op_type)
     cp = _lib.ConvParamsC()
     cp.op_type = int(op)
@@ -111,20 +116,20 @@ def build_conv_params_c(params: ConvParams) -> Tuple[_lib.ConvParamsC, dict]:
     cp.tile_m = int(desp.tile_shape[0])
     cp.tile_k = int(desp.tile_shape[2])
     cp.kv = kv
-    cp.n_in = inp.dim(0)
-    cp.n_out = out.dim(0)
+    cp.n_in = n_in
+    cp.n_out = n_out
     cp.C = C
     cp.K = K
-    cp.N = params.indices.dim(1)
-    cp.input = _ptr(inp)
-    cp.weight = _ptr(w)
-    cp.output = _ptr(out)
-    cp.indices = _ptr(params.indices)
-    cp.mask = _ptr(params.mask)
-    cp.mask_count = params.mask.size
-    cp.mask_argsort = _ptr(params.mask_argsort)
-    cp.mask_output = _ptr(params.mask_output)
-    cp.mask_output_count = params.mask_output.size
+    cp.N = n_rows
+    cp.input = p_inp
+    cp.weight = p_w
+    cp.output = p_out
+    cp.indices = p_indices
+    cp.mask = p_mask
+    cp.mask_count = mask.size
+    cp.mask_argsort = p_argsort
+    cp.mask_output = p_mask_output
+    cp.mask_output_count = mask_output.size
     cp.mask_filter = int(params.mask_filter) & 0xffffffff
     cp.reverse_mask = 1 if params.reverse_mask else 0
     cp.mask_width = int(params.mask_width)
@@ -133,26 +138,23 @@ def build_conv_params_c(params: ConvParams) -> Tuple[_lib.ConvParamsC, dict]:
     cp.act_alpha = float(params.act_alpha)
     cp.act_beta = float(params.act_beta)
     cp.act_type = int(params.act_type)
-    cp.bias = _ptr(params.bias)
-    cp.output_add = _ptr(params.output_add)
-    cp.scale = _ptr(params.scale)
+    cp.bias = p_bias
+    cp.output_add = p_add
+    cp.scale = p_scale
     cp.split_k_slices = int(params.split_k_slices)
     cp.flags = 0
     cp.stream = int(params.stream) if params.stream else None
     isorted = getattr(params, "indices_sorted", None)
     if isorted is not None and not isorted.empty():
-        if list(isorted.shape) != list(params.indices.shape):
+        if isorted._t.shape != indices._t.shape:
             raise ValueError("indices_sorted must have the shape of indices")
-        _check_dense(isorted, "indices_sorted")
-        cp.indices_sorted = isorted.byte_pointer()
+        cp.indices_sorted = _dense_ptr(isorted, "indices_sorted")
     cp.tile_n = int(getattr(params, "tile_n", 0) or 0)
     torder = getattr(params, "tile_order", None)
     if torder is not None and not torder.empty():
-        n_rows = int(params.indices.shape[1])
-        if torder.dtype != tv.int32 or list(torder.shape) != [(n_rows + 127) // 128]:
+        if torder.dtype != tv.int32 or torder.shape != [(n_rows + 127) // 128]:
             raise ValueError("tile_order must be int32 [ceil(N / 128)]")
-        _check_dense(torder, "tile_order")
-        cp.tile_order = torder.byte_pointer()
+        cp.tile_order = _dense_ptr(torder, "tile_order")
     return cp, {"kv": kv, "C": C, "K": K}
 
 

@@ -34,13 +34,17 @@ def _vp(t: torch.Tensor):
     return ctypes.c_void_p(t.data_ptr()) if t is not None and t.numel() > 0 else None
 
 
-def _i32x3(v: Sequence[int]) -> torch.Tensor:
-    return torch.tensor(list(v), dtype=torch.int32)
+_I32x3 = ctypes.c_int32 * 3
+
+
+def _i32x3(v: Sequence[int]):
+    """Three ints as a host array (an argument of the C entry points)."""
+    a, b, c = v
+    return _I32x3(int(a), int(b), int(c))
 
 
 def _stream(stream: int):
-    return ctypes.c_void_p(stream) if stream else (
-        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    return ctypes.c_void_p(stream if stream else _lib.current_stream())
 
 
 def _ws(nbytes: int, device) -> torch.Tensor:
@@ -81,8 +85,7 @@ class SpconvOps:
         mask_full = masks[0] if direct else torch.empty(n, dtype=torch.int32, device=dev)
         s = _stream(stream)
         _lib.check(lib.sc_build_subm_pairs(
-            _vp(coords), n, ctypes.c_void_p(sp.data_ptr()), ctypes.c_void_p(ks.data_ptr()),
-            ctypes.c_void_p(dl.data_ptr()), _vp(pairs[0]), _vp(pairs[1]), _vp(mask_full), _vp(ws),
+            _vp(coords), n, sp, ks, dl, _vp(pairs[0]), _vp(pairs[1]), _vp(mask_full), _vp(ws),
             ws.numel(), s))
         if split_masks is None:
             if not direct:
@@ -113,14 +116,11 @@ class SpconvOps:
         ws = _ws(need.value, dev)
         sp, ks, st, pd, dl = (_i32x3(spatial_shape), _i32x3(ksize), _i32x3(stride), _i32x3(padding),
                               _i32x3(dilation))
-        out_sp = torch.zeros(3, dtype=torch.int32)
+        out_sp = _I32x3()
         n_out = ctypes.c_int64(0)
         s = _stream(stream)
-        args = (ctypes.c_void_p(sp.data_ptr()), ctypes.c_void_p(ks.data_ptr()),
-                ctypes.c_void_p(st.data_ptr()), ctypes.c_void_p(pd.data_ptr()),
-                ctypes.c_void_p(dl.data_ptr()))
-        _lib.check(lib.sc_build_conv_outputs(_vp(coords), n, batch_size, *args,
-                                             ctypes.c_void_p(out_sp.data_ptr()),
+        args = (sp, ks, st, pd, dl)
+        _lib.check(lib.sc_build_conv_outputs(_vp(coords), n, batch_size, *args, out_sp,
                                              ctypes.byref(n_out), _vp(ws), ws.numel(), s))
         no = int(n_out.value)
         out_inds = torch.empty((no, 4), dtype=torch.int32, device=dev)
@@ -131,7 +131,7 @@ class SpconvOps:
         _lib.check(lib.sc_build_conv_pairs(_vp(coords), n, batch_size, *args, no, _vp(out_inds),
                                            _vp(pf), _vp(pb), _vp(mf), _vp(mb), _vp(ws), ws.numel(),
                                            s))
-        return out_inds, pf, pb, mf, mb, [int(x) for x in out_sp]
+        return out_inds, pf, pb, mf, mb, list(out_sp)
 
     @staticmethod
     def sort_1d_by_key_split(data, mask, stream: int = 0):

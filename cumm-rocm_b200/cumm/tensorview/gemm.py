@@ -220,28 +220,31 @@ class ConvAlgoDesp(GemmAlgoDesp):
         self.is_int8_inference = False
         self.dynamic_mask = False
 
+    # operand (0 a, 1 b, 2 c) of input, weight and output per op type
+    _IWO = ((0, 1, 2), (2, 1, 0), (1, 2, 0))
+
     @staticmethod
     def conv_iwo_012_to_abc(op_type: ConvOpType) -> List[int]:
-        return {0: [0, 1, 2], 1: [2, 1, 0], 2: [1, 2, 0]}[int(op_type)]
+        return list(ConvAlgoDesp._IWO[int(op_type)])
 
     @staticmethod
     def gemm_abc_012_to_iwo(op_type: ConvOpType) -> List[int]:
         return {0: [0, 1, 2], 1: [2, 1, 0], 2: [2, 0, 1]}[int(op_type)]
 
     def _abc(self):
-        return [self.dtype_a, self.dtype_b, self.dtype_c]
+        return (self.dtype_a, self.dtype_b, self.dtype_c)
 
     @property
     def dtype_input(self) -> int:
-        return self._abc()[self.conv_iwo_012_to_abc(self.op_type)[0]]
+        return self._abc()[self._IWO[self.op_type][0]]
 
     @property
     def dtype_weight(self) -> int:
-        return self._abc()[self.conv_iwo_012_to_abc(self.op_type)[1]]
+        return self._abc()[self._IWO[self.op_type][1]]
 
     @property
     def dtype_output(self) -> int:
-        return self._abc()[self.conv_iwo_012_to_abc(self.op_type)[2]]
+        return self._abc()[self._IWO[self.op_type][2]]
 
     def __repr__(self) -> str:
         s = super().__repr__()
@@ -373,18 +376,33 @@ class GemmParams:
         self._d = v
 
 
+_EMPTY = None
+
+
+def _empty_tensor():
+    global _EMPTY
+    if _EMPTY is None:
+        from . import Tensor
+        _EMPTY = Tensor()
+    return _EMPTY
+
+
 class ConvParams:
     """Mirror of tv::gemm::ConvParams (params.h:392-428)."""
 
     def __init__(self, ndim: int, op_type: ConvOpType, timer=None):
-        from . import Tensor
-        self.conv_algo_desp = ConvAlgoDesp(ndim, op_type)
-        self.input = Tensor()
-        self.weight = Tensor()
-        self.output = Tensor()
-        self.output_add = Tensor()
-        self.bias = Tensor()
-        self.scale = Tensor()
+        # callers set the descriptor and most tensors right away: the default
+        # descriptor is made when it is read, and unset tensors share one
+        # (immutable) empty wrapper
+        self._desp = None
+        self._desp_args = (ndim, ConvOpType(op_type))
+        none = _empty_tensor()
+        self.input = none
+        self.weight = none
+        self.output = none
+        self.output_add = none
+        self.bias = none
+        self.scale = none
         self.split_k_slices = 1
         self.padding: List[int] = []
         self.stride: List[int] = []
@@ -400,20 +418,30 @@ class ConvParams:
         self.verbose = False
         self.mask_int_count = 1
         self.timer = timer
-        self.workspace = Tensor()
-        self.mask = Tensor()
-        self.mask_argsort = Tensor()
-        self.indices = Tensor()
-        self.mask_output = Tensor()
+        self.workspace = none
+        self.mask = none
+        self.mask_argsort = none
+        self.indices = none
+        self.mask_output = none
         self.stream = 0
         # extension (no counterpart in the reference): indices permuted into
         # mask_argsort order (SpconvOps.sort_indices); lets the kernels read
         # the index table coalesced; results are identical
-        self.indices_sorted = Tensor()
+        self.indices_sorted = none
         # extension: output-column tile of the tcgen05 fwd / dgrad kernels
         # (0 = widest); set by cumm.autotune, results are identical
         self.tile_n = 0
         # extension: the order in which the tcgen05 fwd / dgrad kernels take
         # their 128-row tiles (SpconvOps.tile_order, heaviest first); without
         # it each call computes that order; results are identical
-        self.tile_order = Tensor()
+        self.tile_order = none
+
+    @property
+    def conv_algo_desp(self) -> ConvAlgoDesp:
+        if self._desp is None:
+            self._desp = ConvAlgoDesp(*self._desp_args)
+        return self._desp
+
+    @conv_algo_desp.setter
+    def conv_algo_desp(self, v: ConvAlgoDesp):
+        self._desp = v
