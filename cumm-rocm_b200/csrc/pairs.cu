@@ -95,8 +95,12 @@ __device__ __forceinline__ long long lin_key(int b, int z, int y, int x, const i
 // Hash table over groups of four voxels consecutive in x: one 32-byte slot
 // (one L2 sector) holds the group's key and the index of each of its voxels
 // (-1 = none), so a row of three x-neighbours takes one or two probes instead
-// of three, each probe one sector, and the 0xff fill that empties the keys
-// also empties the indices.
+// of three.  A group lives in the bucket of eight slots that its hash names
+// (where that is full, in the next one with room), and a byte per slot holds
+// seven more bits of the hash: a lookup compares a bucket's eight bytes at once
+// and reads a slot only where one matches, so absent neighbours (most rows off
+// a surface) and other groups' slots cost no slot reads and no probe chains.
+// One 0xff fill empties keys, indices and bytes.
 struct __align__(32) GroupSlot {
   unsigned long long key;  // ((b * D + z) * H + y) * ceil(W / 4) + x / 4; ~0 = empty
   unsigned long long pad;
@@ -104,20 +108,29 @@ struct __align__(32) GroupSlot {
 };
 struct GroupTable {
   GroupSlot *slot;
-  int64_t cap;             // power of two, > 1.5 x voxels, <= 2^32
+  uint8_t *tag;            // 0xff = empty
+  int64_t cap;             // power of two, >= 8, > 1.5 x voxels, <= 2^32
   int log2cap;
 };
 
-// The slot that a key's probing starts at: a 32-bit multiplicative hash of the
-// folded key (neighbouring rows and groups differ in its low bits, which the
-// multiplications carry to the top).  Six instructions: the 64-bit finaliser's
-// twenty were most of the lookups' cost.
-__device__ __forceinline__ uint32_t group_slot(const GroupTable &t, unsigned long long key) {
+// A 32-bit multiplicative hash of the folded key (neighbouring rows and groups
+// differ in its low bits, which the multiplications carry to the top): the top
+// bits name the slot that an insertion starts at, the low seven are the tag.
+// Six instructions: a 64-bit finaliser's twenty were most of the lookups' cost.
+__device__ __forceinline__ uint32_t group_hash(unsigned long long key) {
   uint32_t h = static_cast<uint32_t>(key) + static_cast<uint32_t>(key >> 32) * 0x85ebca6bu;
   h *= 0x9e3779b1u;
   h ^= h >> 15;
-  h *= 0x2c1b3c6du;
-  return h >> (32 - t.log2cap);
+  return h * 0x2c1b3c6du;
+}
+
+// First slot (0..7) of a bucket whose tag matches, -1 if none, with the
+// bucket's tags `g`; `open`: the bucket has an empty slot.
+__device__ __forceinline__ int match_tags(const uint2 &g, uint32_t hash, bool *open) {
+  const uint32_t want = (hash & 127u) * 0x01010101u;
+  const uint32_t lo = __vcmpeq4(g.x, want), hi = __vcmpeq4(g.y, want);
+  *open = (__vcmpeq4(g.x, 0xffffffffu) | __vcmpeq4(g.y, 0xffffffffu)) != 0u;
+  return lo ? (__ffs(lo) - 1) >> 3 : hi ? 4 + ((__ffs(hi) - 1) >> 3) : -1;
 }
 
 __device__ __forceinline__ int4 load_coord(const int32_t *coords, int64_t i, bool vec) {
@@ -139,14 +152,24 @@ insert_groups(const int32_t *coords, int vec, int64_t n, Geom g, GroupTable t, i
   const unsigned long long key = in ? static_cast<unsigned long long>(lin_key(c.x, c.y, c.z, c.w >> 2, gsp)) : ~0ull;
   const unsigned long long prev_key = __shfl_up_sync(0xffffffffu, key, 1);
   const bool leader = lane == 0 || prev_key != key;
-  uint32_t at = group_slot(t, key);
+  const uint32_t hash = group_hash(key);
+  uint32_t at = hash >> (32 - t.log2cap);
   bool placed = false;
   if (leader && in) {
+    // the bucket's eight slots from the hashed one round, then the next bucket
+    const uint32_t start = at & 7u;
+    uint32_t bucket = at & ~7u;
     for (int64_t step = 0; step < t.cap; ++step) {
+      at = bucket | ((start + static_cast<uint32_t>(step)) & 7u);
       const unsigned long long was = atomicCAS(&t.slot[at].key, ~0ull, key);
       placed = was == ~0ull || was == key;
-      if (placed) break;
-      at = (at + 1) & static_cast<uint32_t>(t.cap - 1);
+      if (placed) {
+        // the tag's byte was 0xff, or holds this tag already
+        const uint32_t sh = (at & 3u) * 8u;
+        atomicAnd(reinterpret_cast<uint32_t *>(t.tag) + (at >> 2), ~((~hash & 0xffu | 0x80u) << sh));
+        break;
+      }
+      if ((step & 7) == 7) bucket = (bucket + 8u) & static_cast<uint32_t>(t.cap - 1);
     }
     if (!placed) atomicOr(err, kErrHashFull);
   }
@@ -166,13 +189,21 @@ __device__ __forceinline__ void load_slot(const GroupSlot *s, unsigned long long
   v = make_int4(static_cast<int>(lo), static_cast<int>(lo >> 32), static_cast<int>(hi), static_cast<int>(hi >> 32));
 }
 
-// The slot of group `key` past the one its hash names; null if it is not there.
-__device__ __forceinline__ const GroupSlot *find_group(const GroupTable &t, unsigned long long key, uint32_t at) {
-  for (int64_t step = 1; step < t.cap; ++step) {
-    at = (at + 1) & static_cast<uint32_t>(t.cap - 1);
-    const unsigned long long k = t.slot[at].key;
-    if (k == key) return t.slot + at;
-    if (k == ~0ull) break;
+// The slot of group `key`; null if it is not there.
+__device__ __forceinline__ const GroupSlot *find_group(const GroupTable &t, unsigned long long key) {
+  const uint32_t hash = group_hash(key);
+  const uint32_t want = (hash & 127u) * 0x01010101u;
+  uint32_t bucket = (hash >> (32 - t.log2cap)) & ~7u;
+  for (int64_t step = 0; step < t.cap; step += 8) {
+    const uint2 g = *reinterpret_cast<const uint2 *>(t.tag + bucket);
+    for (int half = 0; half < 2; ++half) {
+      for (uint32_t m = __vcmpeq4(half ? g.y : g.x, want) & 0x01010101u; m != 0u; m &= m - 1u) {
+        const GroupSlot *s = t.slot + bucket + half * 4 + ((__ffs(m) - 1) >> 3);
+        if (s->key == key) return s;
+      }
+    }
+    if ((__vcmpeq4(g.x, 0xffffffffu) | __vcmpeq4(g.y, 0xffffffffu)) != 0u) break;
+    bucket = (bucket + 8u) & static_cast<uint32_t>(t.cap - 1);
   }
   return nullptr;
 }
@@ -191,10 +222,10 @@ __device__ __forceinline__ int pick(const int4 &v, int q) {
 //
 // 3x3x3, dilation 1 (kNine): per z plane the three rows' probes, and those of
 // the second group of lanes at a group's edge, are in flight together.  Bound
-// by the round trips of the probes that go on past their first slot, then by
-// its table writes (216 bytes per voxel).  Both tables, with the fill that the
-// scatter needed: 200k voxels 79 us with 27 chained probes, now 25; 2.6M
-// voxels 600 us, now 409.
+// by two dependent round trips per plane (tags, slots) and by its table writes
+// (216 bytes per voxel).  Both tables, 200k / 2.6M voxels: 79 / 600 us with 27
+// chained hash probes, a fill and a scatter; 25 / 404 with groups and linear
+// probing of the slots; 23 / 263 with tags.
 template <bool kNine>
 __global__ void __launch_bounds__(128)
 subm_pairs_kernel(const int32_t *coords, int vec, int64_t n, Geom g, GroupTable t, int32_t *pairs_fwd,
@@ -226,38 +257,57 @@ subm_pairs_kernel(const int32_t *coords, int vec, int64_t n, Geom g, GroupTable 
     const long long dz = static_cast<long long>(g.spatial[1]) * ng;
     __shared__ int sj[27][128];  // [offset][thread]
     const int tid = threadIdx.x;
-    // Probes whose slot holds another group (a few lanes of most warps): they
-    // probe on together after the straight pass, one each at a time.  Where
-    // each of the 18 steps waited for its own, that was most of the kernel.
+    // Lookups that a bucket's tags do not settle (a full bucket, two groups with
+    // one tag): looked up again after the straight pass, one at a time.
     uint32_t unresolved = 0u;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const bool ok_z = z + a - 1 >= 0 && z + a - 1 < g.spatial[0];
-      unsigned long long k_main[3], f_main[3], f_side[3];
+      unsigned long long k_main[3];
+      uint32_t h_main[3], h_side[3];
+      uint2 g_main[3], g_side[3];
+      bool ok[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        ok[c] = ok_z && y + c - 1 >= 0 && y + c - 1 < g.spatial[1];
+        const unsigned long long k = key0 + static_cast<unsigned long long>((a - 1) * dz + static_cast<long long>(c - 1) * ng);
+        k_main[c] = k;
+        h_main[c] = group_hash(k);
+        h_side[c] = group_hash(k + static_cast<unsigned long long>(static_cast<long long>(side)));
+        g_main[c] = g_side[c] = make_uint2(0xffffffffu, 0xffffffffu);
+        if (ok[c] && has_main)
+          g_main[c] = __ldg(reinterpret_cast<const uint2 *>(t.tag + ((h_main[c] >> (32 - t.log2cap)) & ~7u)));
+        if (ok[c] && has_side)
+          g_side[c] = __ldg(reinterpret_cast<const uint2 *>(t.tag + ((h_side[c] >> (32 - t.log2cap)) & ~7u)));
+      }
+      unsigned long long f_main[3], f_side[3];
       int4 v[3];
       int vs[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const bool ok = ok_z && y + c - 1 >= 0 && y + c - 1 < g.spatial[1];
-        const unsigned long long k = key0 + static_cast<unsigned long long>((a - 1) * dz + static_cast<long long>(c - 1) * ng);
-        k_main[c] = k;
-        f_main[c] = f_side[c] = ~0ull;
+        f_main[c] = k_main[c];
+        f_side[c] = k_main[c] + static_cast<unsigned long long>(static_cast<long long>(side));
         v[c] = make_int4(-1, -1, -1, -1);
         vs[c] = -1;
-        if (ok && has_main) {
-          load_slot(t.slot + group_slot(t, k), f_main[c], v[c]);
-        }
-        if (ok && has_side) {
-          const GroupSlot *s = t.slot + group_slot(t, k + static_cast<unsigned long long>(static_cast<long long>(side)));
+        bool open;
+        int at = match_tags(g_main[c], h_main[c], &open);
+        if (at >= 0)
+          load_slot(t.slot + ((h_main[c] >> (32 - t.log2cap)) & ~7u) + at, f_main[c], v[c]);
+        else if (!open)
+          unresolved |= 1u << (a * 3 + c);
+        at = match_tags(g_side[c], h_side[c], &open);
+        if (at >= 0) {
+          const GroupSlot *s = t.slot + ((h_side[c] >> (32 - t.log2cap)) & ~7u) + at;
           f_side[c] = s->key;
           vs[c] = s->v[side < 0 ? 3 : 0];
+        } else if (!open) {
+          unresolved |= 512u << (a * 3 + c);
         }
       }
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        // an empty slot holds -1 throughout
-        if (f_main[c] != k_main[c] && f_main[c] != ~0ull) unresolved |= 1u << (a * 3 + c);
-        if (f_side[c] != k_main[c] + static_cast<unsigned long long>(static_cast<long long>(side)) && f_side[c] != ~0ull)
+        if (f_main[c] != k_main[c]) unresolved |= 1u << (a * 3 + c);
+        if (f_side[c] != k_main[c] + static_cast<unsigned long long>(static_cast<long long>(side)))
           unresolved |= 512u << (a * 3 + c);
         const int beside_up = __shfl_up_sync(0xffffffffu, v[c].w, 1);
         const int beside_dn = __shfl_down_sync(0xffffffffu, v[c].x, 1);
@@ -281,7 +331,7 @@ subm_pairs_kernel(const int32_t *coords, int vec, int64_t n, Geom g, GroupTable 
       const int r = is_side ? b - 9 : b;
       const unsigned long long key = key0 + static_cast<unsigned long long>(
           (r / 3 - 1) * dz + static_cast<long long>(r % 3 - 1) * ng + (is_side ? side : 0));
-      const GroupSlot *s = find_group(t, key, group_slot(t, key));
+      const GroupSlot *s = find_group(t, key);
       if (is_side) {
         sj[r * 3 + (side < 0 ? 0 : 2)][tid] = s ? s->v[side < 0 ? 3 : 0] : -1;
       } else {
@@ -306,11 +356,7 @@ subm_pairs_kernel(const int32_t *coords, int vec, int64_t n, Geom g, GroupTable 
     auto lookup = [&](int zz, int yy, int xx) {
       if (zz < 0 || yy < 0 || xx < 0 || zz >= g.spatial[0] || yy >= g.spatial[1] || xx >= g.spatial[2]) return -1;
       const unsigned long long key = static_cast<unsigned long long>(lin_key(co.x, zz, yy, xx >> 2, gsp));
-      const uint32_t at = group_slot(t, key);
-      const GroupSlot *s = t.slot + at;
-      const unsigned long long first = s->key;
-      if (first == ~0ull) return -1;
-      if (first != key) s = find_group(t, key, at);
+      const GroupSlot *s = find_group(t, key);
       return s ? s->v[xx & 3] : -1;
     };
     const bool held = lookup(z, y, x) == static_cast<int>(i);
@@ -1020,7 +1066,7 @@ int64_t conv_bytes(int64_t n_in, int kv) {
   return h > kMinMapBytes ? h : kMinMapBytes;
 }
 
-int64_t group_cap(int64_t n) { return next_pow2(n + n / 2 + 1); }
+int64_t group_cap(int64_t n) { return next_pow2(n + n / 2 + 8); }
 
 int64_t map_cells(const Geom &g, int64_t batch) {
   const double est = static_cast<double>(batch) * g.out_spatial[0] * g.out_spatial[1] * g.out_spatial[2];
@@ -1042,7 +1088,7 @@ bool map_fits(int64_t cells, int64_t n_in, int kv) {
 
 int64_t pairs_workspace_bytes(int64_t n_in, int kv, int subm) {
   // 512: the head of a strided build and the alignment of the pointer given
-  if (subm) return group_cap(n_in) * static_cast<int64_t>(sizeof(GroupSlot)) + 512;
+  if (subm) return group_cap(n_in) * (static_cast<int64_t>(sizeof(GroupSlot)) + 1) + 512;
   return conv_bytes(n_in, kv) + 512;
 }
 
@@ -1081,7 +1127,8 @@ cudaError_t build_subm_pairs(const PairBuildArgs &a, int32_t *pairs_fwd, int32_t
   t.log2cap = 63 - __builtin_clzll(static_cast<unsigned long long>(t.cap));
   t.slot = reinterpret_cast<GroupSlot *>(align_ptr(ws));
   const int vec = reinterpret_cast<uintptr_t>(a.coords) % 16 == 0;
-  cudaError_t e = cudaMemsetAsync(t.slot, 0xff, t.cap * sizeof(GroupSlot), s);
+  t.tag = reinterpret_cast<uint8_t *>(t.slot + t.cap);
+  cudaError_t e = cudaMemsetAsync(t.slot, 0xff, t.cap * (sizeof(GroupSlot) + 1), s);
   if (e != cudaSuccess) return e;
   insert_groups<<<blocks_of(n, kThreads), kThreads, 0, s>>>(a.coords, vec, n, g, t, a.err);
   bool nine = true;
