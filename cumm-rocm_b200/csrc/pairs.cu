@@ -771,7 +771,7 @@ __global__ void radix_scatter(const K *keys, const int32_t *vals, K *keys_out, i
 // own launch and scanned by another: there the reductions cost more than those
 // (2.6M rows: 43 us a pass with them, 23 + 9 + 4 without).
 // Per pass, against a histogram, a one-block scan and a match_any scatter:
-// 200k rows 36 -> 11 us, 60k rows 26 -> 5, 2.6M rows 148 -> 36.
+// 200k rows 36 -> 10 us, 60k rows 26 -> 5, 2.6M rows 148 -> 36.
 constexpr int kMaskThreads = 256;
 constexpr int kMaskWarps = kMaskThreads / 32;
 constexpr int kMaskBins = 256;
@@ -960,8 +960,9 @@ MaskSort mask_sort_plan(int64_t n, uint32_t split) {
   P.passes = (bits + 7) / 8;
   P.bits = (bits + P.passes - 1) / P.passes;
   // Small tiles while that keeps the count rows short: more blocks, fewer
-  // serial rounds per warp.
-  P.tile_shift = n <= (int64_t(kMaskRowTiles) << 10) ? 10 : 11;
+  // serial rounds per warp, against more rows for every tile to sum (200k rows
+  // a pass: 11.3 us with 196 tiles, 10.1 with 98).
+  P.tile_shift = n <= (int64_t(kMaskRowTiles) << 10) / 2 ? 10 : 11;
   P.tiles = static_cast<int>((n + (int64_t(1) << P.tile_shift) - 1) >> P.tile_shift);
   P.pitch = (P.tiles + 3) & ~3;
   return P;
