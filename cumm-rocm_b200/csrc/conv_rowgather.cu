@@ -262,24 +262,6 @@ __device__ __forceinline__ void store_row(TOut *p, const float *v) {
   }
 }
 
-// The activation of n values.  One branch on the type for all of them: with the
-// switch inside the loop every element branched, 2,100 cycles per 16 columns of
-// a tile and more than half of the epilogue warps' time.
-template <int n>
-__device__ __forceinline__ void apply_act_n(float *v, int type, float a) {
-  if (type == 0) return;
-  if (type == 1) {
-#pragma unroll
-    for (int i = 0; i < n; ++i) v[i] = apply_act(v[i], 1, a);
-  } else if (type == 2) {
-#pragma unroll
-    for (int i = 0; i < n; ++i) v[i] = apply_act(v[i], 2, a);
-  } else if (type == 3) {
-#pragma unroll
-    for (int i = 0; i < n; ++i) v[i] = apply_act(v[i], 3, a);
-  }
-}
-
 // Applies the epilogue to `n` (16 or 32) consecutive columns starting at column
 // `col` of output row `orow` and stores them.
 template <int n, typename TOut>

@@ -13,11 +13,11 @@
 // 2-D TMA boxes into a 4-stage ring (48 KB per stage, SWIZZLE_128B); a
 // row-major operand is K-major for the tensor core and a transposed one is
 // read in place as MN-major (no copy).  Warp 5 issues tcgen05.mma (M = 128,
-// N = 256, K = 16; one issuing warp completes such an MMA about as fast as
-// the tensor pipe runs it) into a double-buffered 128 x 256 fp32 TMEM
+// N = 256, K = 16, 128 cycles each from one issuing thread: the tensor pipe's
+// rate) into a double-buffered 128 x 256 fp32 TMEM
 // accumulator, so warps 0-3 run the epilogue of one tile while the next one
 // accumulates.  The epilogue applies act(alpha acc + beta D) and stores
-// 32-byte row segments, or with split-K adds its partial tile into an fp32
+// whole 128-byte lines, or with split-K adds its partial tile into an fp32
 // workspace with red.global.add.v4.f32 (a finalize pass applies the
 // epilogue).  Rows and columns past m / n / k are TMA zero fill on the loads
 // and skipped on the stores.  Every mbarrier wait is bounded.
@@ -31,6 +31,7 @@ namespace {
 constexpr int kBM = 128, kBN = 256, kBK = 64;
 constexpr int kStages = 4;
 constexpr int kThreads = 192;  // warps 0-3 epilogue, 4 TMA producer, 5 MMA issuer
+constexpr int kWarpBuf = 4096;  // bytes per epilogue warp: 32 rows x 128 bytes
 constexpr int kGroupM = 16;    // row tiles per raster group
 constexpr uint32_t kABytes = kBM * kBK * 2;  // 16 KB
 constexpr uint32_t kBBytes = kBN * kBK * 2;  // 32 KB
@@ -84,17 +85,38 @@ __device__ __forceinline__ void red_add_v4(float *p, float a, float b, float c, 
                : "memory");
 }
 
-__device__ __forceinline__ void st_global_v8(void *p, const uint32_t *w) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]),
-               "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-               : "memory");
+// act(alpha acc + beta D) of `ncol` (16: all) columns from col0 of output row `row`.
+template <typename TOut>
+__device__ __forceinline__ void apply16(const GemmArgs &G, int64_t row, int64_t col0, int64_t ncol, float *acc) {
+  const EpiParams &e = G.epi;
+  constexpr int kPer16 = 16 / sizeof(TOut);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) acc[i] *= e.alpha;
+  if (e.beta != 0.f && e.src != nullptr) {
+    const TOut *src = static_cast<const TOut *>(e.src) + row * e.src_ld + col0;
+    if (ncol == 16 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+#pragma unroll
+      for (int i = 0; i < 16; i += kPer16) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(src + i);
+        const TOut *h = reinterpret_cast<const TOut *>(&q);
+#pragma unroll
+        for (int j = 0; j < kPer16; ++j) acc[i + j] = fmaf(e.beta, to_f32(h[j]), acc[i + j]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (i < ncol) acc[i] = fmaf(e.beta, to_f32(src[i]), acc[i]);
+      }
+    }
+  }
+  apply_act_n<16>(acc, e.act_type, e.act_alpha);
 }
 
-// Epilogue of 16 accumulator columns [col0, col0 + 16) of output row `row`.
+// Epilogue of 16 accumulator columns [col0, col0 + 16) of output row `row`,
+// stored (or, with split-K, added) by the row's own thread.
 template <typename TOut>
 __device__ __forceinline__ void store16(const DParams &P, int64_t row, int64_t col0, float *acc) {
   const GemmArgs &G = P.g;
-  const EpiParams &e = G.epi;
   const int64_t ncol = G.n - col0 < 16 ? G.n - col0 : 16;
   if (P.ws != nullptr) {
     float *w = P.ws + row * G.n + col0;
@@ -102,36 +124,78 @@ __device__ __forceinline__ void store16(const DParams &P, int64_t row, int64_t c
 #pragma unroll
       for (int i = 0; i < 16; i += 4) red_add_v4(w + i, acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
     } else {
-      for (int i = 0; i < ncol; ++i) atomicAdd(w + i, acc[i]);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (i < ncol) atomicAdd(w + i, acc[i]);
+      }
     }
     return;
   }
-  const bool use_src = e.beta != 0.f && e.src != nullptr;
-  const TOut *src = use_src ? static_cast<const TOut *>(e.src) + row * e.src_ld + col0 : nullptr;
+  apply16<TOut>(G, row, col0, ncol, acc);
+  TOut *dst = static_cast<TOut *>(G.c) + row * G.ldc + col0;
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    float v = e.alpha * acc[i];
-    if (use_src && i < ncol) v = fmaf(e.beta, to_f32(src[i]), v);
-    acc[i] = apply_act(v, e.act_type, e.act_alpha);
+    if (i < ncol) dst[i] = from_f32<TOut>(acc[i]);
   }
-  TOut *dst = static_cast<TOut *>(G.c) + row * G.ldc + col0;
-  constexpr int kPer32 = 32 / sizeof(TOut);
-  if (ncol == 16 && (reinterpret_cast<uintptr_t>(dst) & 31u) == 0) {
+}
+
+// Epilogue of one warp's 32 rows (from row0, TMEM address t0) x 256 columns
+// from nb.  Column blocks of 128 bytes go through the warp's 4 KB of shared
+// memory (16-byte units XOR-swizzled by row) so that a store instruction
+// writes four whole 128-byte lines; a row per thread wrote 32 pieces of 32
+// lines (16384 x 4096 x 2048: 200 us, staged 187; 8192^3 762 / 750; with K = 256
+// it costs 84 / 86).  Blocks that n cuts, split-K and rows that do not start on
+// 16 bytes are written by the rows' own threads.  With the activation's switch
+// outside the element loop this took 8192 x 8192 x 256 from 367 to 138 us and
+// 304 x 520 x 200 from 48 to 15: a tile's epilogue was longer than its mainloop
+// up to K of about 4096.
+template <typename TOut>
+__device__ __forceinline__ void store_tile(const DParams &P, uint8_t *buf, int lane, int64_t row0, int64_t nb,
+                                           uint32_t t0, bool any) {
+  const GemmArgs &G = P.g;
+  constexpr int kCols = 128 / sizeof(TOut);
+  constexpr int kUnits = 16 * sizeof(TOut) / 16;  // 16-byte units of 16 columns
+  const int64_t row = row0 + lane;
+  const bool lines = P.ws == nullptr && (reinterpret_cast<uintptr_t>(G.c) & 15u) == 0 &&
+                     (G.ldc * static_cast<int64_t>(sizeof(TOut))) % 16 == 0;
+  for (int cb = 0; cb < kBN; cb += kCols) {
+    if (nb + cb >= G.n) break;  // warp-uniform
+    const bool whole = lines && nb + cb + kCols <= G.n;
 #pragma unroll
-    for (int i = 0; i < 16; i += kPer32) {
-      uint32_t w[8];
-      if constexpr (sizeof(TOut) == 4) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) w[j] = __float_as_uint(acc[i + j]);
+    for (int q = 0; q < kCols / 16; ++q) {
+      const int64_t col0 = nb + cb + q * 16;
+      float acc[16];
+      if (any) {
+        tmem_ld16(t0 + static_cast<uint32_t>(cb + q * 16), acc);
       } else {
-        TOut *h = reinterpret_cast<TOut *>(w);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) h[j] = from_f32<TOut>(acc[i + j]);
+        for (int i = 0; i < 16; ++i) acc[i] = 0.f;
       }
-      st_global_v8(dst + i, w);
+      if (!whole) {
+        if (row < G.m && col0 < G.n) store16<TOut>(P, row, col0, acc);
+        continue;
+      }
+      if (row < G.m) apply16<TOut>(G, row, col0, 16, acc);
+#pragma unroll
+      for (int u = 0; u < kUnits; ++u) {
+        uint4 w;
+        TOut *h = reinterpret_cast<TOut *>(&w);
+#pragma unroll
+        for (int j = 0; j < 16 / static_cast<int>(sizeof(TOut)); ++j)
+          h[j] = from_f32<TOut>(acc[u * (16 / sizeof(TOut)) + j]);
+        *reinterpret_cast<uint4 *>(buf + lane * 128 + (((q * kUnits + u) ^ (lane & 7)) << 4)) = w;
+      }
     }
-  } else {
-    for (int i = 0; i < ncol; ++i) dst[i] = from_f32<TOut>(acc[i]);
+    if (!whole) continue;
+    __syncwarp();
+    TOut *dst = static_cast<TOut *>(G.c) + nb + cb + (lane & 7) * (16 / sizeof(TOut));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + (lane >> 3);
+      const uint4 w = *reinterpret_cast<const uint4 *>(buf + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+      if (row0 + r < G.m) *reinterpret_cast<uint4 *>(dst + (row0 + r) * G.ldc) = w;
+    }
+    __syncwarp();
   }
 }
 
@@ -305,19 +369,8 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
       const int64_t tile = u / P.splits;
       int64_t mt, nt;
       tile_mn(P, tile, mt, nt);
-      const int64_t row = mt * kBM + threadIdx.x;
-      const int64_t nb = nt * kBN;
-      for (int cc = 0; cc < kBN; cc += 16) {
-        if (nb + cc >= G.n) break;  // warp-uniform
-        float acc[16];
-        if (nkb > 0) {
-          tmem_ld16(tmem_base + lane_base + static_cast<uint32_t>(ab * kBN + cc), acc);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) acc[i] = 0.f;
-        }
-        if (row < G.m) store16<TOut>(P, row, nb + cc, acc);
-      }
+      store_tile<TOut>(P, smem + kStages * kStageBytes + warp * kWarpBuf, lane, mt * kBM + warp * 32, nt * kBN,
+                       tmem_base + lane_base + static_cast<uint32_t>(ab * kBN), nkb > 0);
       tc_fence_before();
       mbar_arrive(&acc_empty[ab]);
     }
@@ -353,6 +406,12 @@ int dense_gemm_splits(const GemmArgs &a) {
 cudaError_t launch_dense_gemm(const GemmArgs &a, float *split_ws, int num_sms, cudaStream_t stream) {
   DParams P;
   P.g = a;
+  const int splits = dense_gemm_splits(a);
+  const int64_t n_tiles = (a.n + kBN - 1) / kBN;
+  const int64_t units1 = (a.m + kBM - 1) / kBM * n_tiles * splits;
+  P.kblocks = static_cast<int>((a.k + kBK - 1) / kBK);
+  P.splits = splits;
+  P.kb_per_split = P.kblocks > 0 ? (P.kblocks + P.splits - 1) / P.splits : 0;
   P.a_mn = a.trans_a ? 1 : 0;
   P.b_mn = a.trans_b ? 0 : 1;
   // A: [m, k] (K-major, 64 x 128 boxes) or stored [k, m] (MN-major, 64 x 64 boxes)
@@ -368,18 +427,14 @@ cudaError_t launch_dense_gemm(const GemmArgs &a, float *split_ws, int num_sms, c
                            : encode_tmap_2d(&P.tb, a.in_dtype, a.b, static_cast<uint64_t>(a.k > 0 ? a.k : 1),
                                             static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.ldb) * 2, 64, kBN);
   if (!ok_a || !ok_b) return cudaErrorInvalidValue;
-  const int64_t m_tiles = (a.m + kBM - 1) / kBM;
-  P.m_tiles = m_tiles;
-  P.n_tiles = (a.n + kBN - 1) / kBN;
-  P.kblocks = static_cast<int>((a.k + kBK - 1) / kBK);
-  P.splits = dense_gemm_splits(a);
-  P.kb_per_split = P.kblocks > 0 ? (P.kblocks + P.splits - 1) / P.splits : 0;
-  P.units = m_tiles * P.n_tiles * P.splits;
+  P.m_tiles = (a.m + kBM - 1) / kBM;
+  P.n_tiles = n_tiles;
+  P.units = units1;
   P.ws = P.splits > 1 ? split_ws : nullptr;
-  P.bar_off = kStages * kStageBytes;
+  P.bar_off = kStages * kStageBytes + 4 * kWarpBuf;
   P.idesc = make_idesc(kBM, kBN, a.in_dtype == 12 ? 1u : 0u, P.a_mn != 0, P.b_mn != 0);
   const size_t smem = 1024 + P.bar_off + 256;
-  const int grid = static_cast<int>(P.units < num_sms ? P.units : num_sms);
+  const int grid = static_cast<int>(units1 < num_sms ? units1 : num_sms);
   void (*kern)(DParams);
   switch (a.out_dtype) {
     case 0: kern = dense_gemm_kernel<float>; break;
