@@ -8,8 +8,10 @@
 // split-K as in cumm/gemm/nvrtc_code.py:68-75 and params.h:115-132, here as a
 // parallel reduction into an fp32 workspace instead of the serial semaphore).
 //
-// B200 design: persistent CTAs (one per SM) walk (128 x 256 output tile,
-// K split) work units.  Warp 4 loads 128 x 64 A and 256 x 64 B blocks with
+// B200 design, two kernels: CTA pairs on 256 x 256 tiles where K is long
+// (dense_gemm_pair_kernel; the rule is in launch_dense_gemm), and single CTAs
+// on 128 x 256 tiles.  The single one: persistent CTAs (one per SM) walk
+// (128 x 256 output tile, K split) work units.  Warp 4 loads 128 x 64 A and 256 x 64 B blocks with
 // 2-D TMA boxes into a 4-stage ring (48 KB per stage, SWIZZLE_128B); a
 // row-major operand is K-major for the tensor core and a transposed one is
 // read in place as MN-major (no copy).  Warp 5 issues tcgen05.mma (M = 128,
@@ -37,6 +39,15 @@ constexpr uint32_t kABytes = kBM * kBK * 2;  // 16 KB
 constexpr uint32_t kBBytes = kBN * kBK * 2;  // 32 KB
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
 
+// CTA-pair kernel: a 256 x 256 tile per pair, 128 rows of A and 128 columns of
+// B loaded by each CTA.  Six stages leave room for the epilogue's buffers; seven
+// without them ran 8192^3 in 715 us against 686.
+constexpr int kPairMinBlocks = 16;
+constexpr int kPairBM = 256;
+constexpr int kPairStages = 6;
+constexpr uint32_t kPairBBytes = kBN / 2 * kBK * 2;  // 16 KB
+constexpr uint32_t kPairStageBytes = kABytes + kPairBBytes;
+
 struct DParams {
   CUtensorMap ta;
   CUtensorMap tb;
@@ -52,15 +63,16 @@ struct DParams {
 __device__ __forceinline__ void flag_error(int *err, int bits) { atomicOr(err, bits); }
 
 // Output tile -> (row tile, column tile).  Tiles are walked in groups of
-// kGroupM row tiles, column by column inside a group, so the tiles that the
+// kGroupM row tiles (half as many of the pair kernel's 256-row tiles), column by column inside a group, so the tiles that the
 // persistent CTAs hold at one time (one each) cover a compact block: at
 // 8192^3, 16 row tiles x ~10 column tiles = 34 MB of A and 42 MB of B, which
 // stay in L2 instead of B streaming from HBM once per 4.6 row tiles.
+template <int kGroup = kGroupM>
 __device__ __forceinline__ void tile_mn(const DParams &P, int64_t tile, int64_t &mt, int64_t &nt) {
-  const int64_t per_group = static_cast<int64_t>(kGroupM) * P.n_tiles;
+  const int64_t per_group = static_cast<int64_t>(kGroup) * P.n_tiles;
   const int64_t g = tile / per_group;
-  const int64_t first = g * kGroupM;
-  const int64_t gm = P.m_tiles - first < kGroupM ? P.m_tiles - first : kGroupM;
+  const int64_t first = g * kGroup;
+  const int64_t gm = P.m_tiles - first < kGroup ? P.m_tiles - first : kGroup;
   const int64_t r = tile - g * per_group;
   mt = first + r % gm;
   nt = r / gm;
@@ -384,6 +396,238 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
   }
 }
 
+// ---- CTA pair (cta_group::2) primitives
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Shared-window address of `addr` in the pair's leader (rank 0).
+__device__ __forceinline__ uint32_t leader_smem(uint32_t addr) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t leader_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_bar) : "memory");
+}
+// 2-D box into this CTA's shared memory; the bytes complete on the leader's barrier.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y,
+                                                 uint32_t leader_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(leader_bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// Arrive on the barrier at this offset in both CTAs once the pair's MMAs so far are done.
+__device__ __forceinline__ void mma_commit_pair(uint64_t *bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
+
+// One 256 x 256 tile per CTA pair (cta_group::2): the tensor core reads both
+// CTAs' B halves, so a CTA stages 32 KB per 64 K-elements instead of 48, moves
+// a third less through L2 and holds six stages instead of four; a pair's MMA
+// (M = 256, N = 256, K = 16) takes the 128 cycles of the single one's
+// M = 128.  Rank 0's MMA warp issues for both; its full barriers count both
+// CTAs' loads, and its commits release the stages of both.  The sums are the
+// single kernel's, in its order.  8192^3: 750 -> 686 us (1,600 TFLOP/s); what
+// is left is the tensor pipe at the clock that the power limit allows, and the
+// last wave (1,024 units on 74 pairs: 13.8 waves).
+template <typename TOut>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+    dense_gemm_pair_kernel(const __grid_constant__ DParams P) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw_u32 = smem_u32(smem_raw);
+  const uint32_t pad = (1024u - (raw_u32 & 1023u)) & 1023u;  // the same in both CTAs
+  uint8_t *smem = smem_raw + pad;
+  const uint32_t smem_base = raw_u32 + pad;
+  const GemmArgs &G = P.g;
+
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + P.bar_off);
+  uint64_t *full = bars;                    // leader's: both CTAs' loads
+  uint64_t *empty = full + kPairStages;     // each CTA's: the pair's MMAs have read the stage
+  uint64_t *acc_full = empty + kPairStages; // each CTA's
+  uint64_t *acc_empty = acc_full + 2;       // leader's: both CTAs' epilogue threads
+  uint64_t *drain_bar = acc_empty + 2;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain_bar + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const int64_t first = blockIdx.x >> 1;
+  const int64_t step = gridDim.x >> 1;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kPairStages; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], 256);
+    }
+    mbar_init(drain_bar, 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 5) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(512)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 4) {
+    // ---------------------------------------------------------------- TMA producer (both CTAs)
+    if (elect_one()) {
+      uint32_t stage = 0, eph = 0;
+      bool ok = true;
+      for (int64_t u = first; u < P.units && ok; u += step) {
+        const int64_t tile = u / P.splits;
+        const int ks = static_cast<int>(u % P.splits);
+        int64_t mt, nt;
+        tile_mn<kGroupM / 2>(P, tile, mt, nt);
+        const int m0 = static_cast<int>(mt * kPairBM) + static_cast<int>(rank) * kBM;
+        const int n0 = static_cast<int>(nt * kBN) + static_cast<int>(rank) * (kBN / 2);
+        const int kb0 = ks * P.kb_per_split;
+        const int kb1 = min(P.kblocks, kb0 + P.kb_per_split);
+        for (int kb = kb0; kb < kb1; ++kb) {
+          if (!mbar_wait(&empty[stage], eph ^ 1u, abort_flag)) {
+            flag_error(G.err, kErrWaitTimeout);
+            ok = false;
+            break;
+          }
+          const uint32_t sA = smem_base + stage * kPairStageBytes;
+          const uint32_t sB = sA + kABytes;
+          const int k0 = kb * kBK;
+          // A peer's bytes may land before the leader expects them: the phase
+          // cannot end before the leader's one arrival.
+          if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2 * kPairStageBytes);
+          const uint32_t bar = leader_smem(smem_u32(&full[stage]));
+          if (P.a_mn) {
+            tma_load_2d_pair(sA, &P.ta, m0, k0, bar);
+            tma_load_2d_pair(sA + 8192, &P.ta, m0 + 64, k0, bar);
+          } else {
+            tma_load_2d_pair(sA, &P.ta, k0, m0, bar);
+          }
+          if (P.b_mn) {
+            tma_load_2d_pair(sB, &P.tb, n0, k0, bar);
+            tma_load_2d_pair(sB + 8192, &P.tb, n0 + 64, k0, bar);
+          } else {
+            tma_load_2d_pair(sB, &P.tb, k0, n0, bar);
+          }
+          if (++stage == kPairStages) {
+            stage = 0;
+            eph ^= 1u;
+          }
+        }
+      }
+    }
+  } else if (warp == 5) {
+    // ---------------------------------------------------------------- MMA issuer (leader only)
+    if (rank == 0 && elect_one()) {
+      uint32_t stage = 0, fph = 0;
+      bool ok = true;
+      int it = 0;
+      for (int64_t u = first; u < P.units && ok; u += step, ++it) {
+        const int ab = it & 1;
+        const uint32_t aph = (it >> 1) & 1;
+        if (!mbar_wait(&acc_empty[ab], aph ^ 1u, abort_flag)) {
+          flag_error(G.err, kErrWaitTimeout);
+          break;
+        }
+        tc_fence_after();
+        const int kb0 = static_cast<int>(u % P.splits) * P.kb_per_split;
+        const int nkb = max(0, min(P.kblocks, kb0 + P.kb_per_split) - kb0);
+        const uint32_t d = tmem_base + static_cast<uint32_t>(ab * kBN);
+        for (int j = 0; j < nkb; ++j) {
+          if (!mbar_wait(&full[stage], fph, abort_flag)) {
+            flag_error(G.err, kErrWaitTimeout);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t sA = smem_base + stage * kPairStageBytes;
+          const uint32_t sB = sA + kABytes;
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            const uint64_t ad = P.a_mn ? make_sdesc(sA + kk * 2048, 8192, 1024) : make_sdesc(sA + kk * 32, 16, 1024);
+            const uint64_t bd = P.b_mn ? make_sdesc(sB + kk * 2048, 8192, 1024) : make_sdesc(sB + kk * 32, 16, 1024);
+            mma_f16_pair(d, ad, bd, P.idesc, (j | kk) != 0 ? 1u : 0u);
+          }
+          mma_commit_pair(&empty[stage]);
+          if (++stage == kPairStages) {
+            stage = 0;
+            fph ^= 1u;
+          }
+        }
+        if (ok) mma_commit_pair(&acc_full[ab]);
+      }
+      mma_commit_pair(drain_bar);
+    }
+    __syncwarp();
+  } else {
+    // ---------------------------------------------------------------- epilogue (warps 0-3, both CTAs)
+    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+    int it = 0;
+    for (int64_t u = first; u < P.units; u += step, ++it) {
+      const int ab = it & 1;
+      const uint32_t aph = (it >> 1) & 1;
+      const int64_t tile = u / P.splits;
+      const int kb0 = static_cast<int>(u % P.splits) * P.kb_per_split;
+      const bool any = kb0 < P.kblocks;
+      if (!mbar_wait(&acc_full[ab], aph, abort_flag)) {
+        flag_error(G.err, kErrWaitTimeout);
+        break;
+      }
+      tc_fence_after();
+      int64_t mt, nt;
+      tile_mn<kGroupM / 2>(P, tile, mt, nt);
+      store_tile<TOut>(P, smem + kPairStages * kPairStageBytes + warp * kWarpBuf, lane,
+                       mt * kPairBM + static_cast<int64_t>(rank) * kBM + warp * 32, nt * kBN,
+                       tmem_base + lane_base + static_cast<uint32_t>(ab * kBN), any);
+      tc_fence_before();
+      mbar_arrive_leader(leader_smem(smem_u32(&acc_empty[ab])));
+    }
+  }
+
+  // Neither CTA leaves while the pair's MMAs may still read its shared memory,
+  // write its TMEM or signal its barriers; every wait is bounded, so both come here.
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int never = 0;
+    if (!mbar_wait(drain_bar, 0, reinterpret_cast<volatile int *>(&never))) flag_error(G.err, kErrWaitTimeout);
+  }
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 5) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
+  }
+}
+
 }  // namespace
 
 bool dense_gemm_supported(const GemmArgs &a) {
@@ -409,9 +653,21 @@ cudaError_t launch_dense_gemm(const GemmArgs &a, float *split_ws, int num_sms, c
   const int splits = dense_gemm_splits(a);
   const int64_t n_tiles = (a.n + kBN - 1) / kBN;
   const int64_t units1 = (a.m + kBM - 1) / kBM * n_tiles * splits;
+  const int64_t units2 = (a.m + kPairBM - 1) / kPairBM * n_tiles * splits;
   P.kblocks = static_cast<int>((a.k + kBK - 1) / kBK);
   P.splits = splits;
   P.kb_per_split = P.kblocks > 0 ? (P.kblocks + P.splits - 1) / P.splits : 0;
+  // CTA pairs where the mainloop is long enough to bound a tile: K >= 1024 per
+  // unit.  us, single / pair: 8192 x 8192 x K with K = 512: 90 / 96, 1024:
+  // 104 / 104, 1536: 144 / 125, 2048: 188 / 158; 60000 x 512 x K: 51 / 53,
+  // 66 / 64, 86 / 76, 107 / 92; 256 x 8192 x K: 16 / 18, 21 / 21, 25 / 23,
+  // 27 / 25.  Below that the epilogue bounds the tile, and the pair's two
+  // epilogues wait for each other.  And only where 256-row tiles take no more
+  // waves: 1152 x 8192 x 4096 is 288 units in 2 waves of 148, or 160 in 3 waves
+  // of 74 (68 / 76); 1280 rows take 3 either way (95 / 79).
+  const int pairs = num_sms / 2;
+  const bool pair = P.kb_per_split >= kPairMinBlocks && pairs > 0 &&
+                    (units2 + pairs - 1) / pairs <= (units1 + num_sms - 1) / num_sms;
   P.a_mn = a.trans_a ? 1 : 0;
   P.b_mn = a.trans_b ? 0 : 1;
   // A: [m, k] (K-major, 64 x 128 boxes) or stored [k, m] (MN-major, 64 x 64 boxes)
@@ -425,21 +681,22 @@ cudaError_t launch_dense_gemm(const GemmArgs &a, float *split_ws, int num_sms, c
                                             static_cast<uint64_t>(a.k > 0 ? a.k : 1),
                                             static_cast<uint64_t>(a.ldb) * 2, 64, 64)
                            : encode_tmap_2d(&P.tb, a.in_dtype, a.b, static_cast<uint64_t>(a.k > 0 ? a.k : 1),
-                                            static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.ldb) * 2, 64, kBN);
+                                            static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.ldb) * 2, 64, pair ? kBN / 2 : kBN);
   if (!ok_a || !ok_b) return cudaErrorInvalidValue;
-  P.m_tiles = (a.m + kBM - 1) / kBM;
+  P.m_tiles = pair ? (a.m + kPairBM - 1) / kPairBM : (a.m + kBM - 1) / kBM;
   P.n_tiles = n_tiles;
-  P.units = units1;
+  P.units = pair ? units2 : units1;
   P.ws = P.splits > 1 ? split_ws : nullptr;
-  P.bar_off = kStages * kStageBytes + 4 * kWarpBuf;
-  P.idesc = make_idesc(kBM, kBN, a.in_dtype == 12 ? 1u : 0u, P.a_mn != 0, P.b_mn != 0);
+  P.bar_off = (pair ? kPairStages * kPairStageBytes : kStages * kStageBytes) + 4 * kWarpBuf;
+  P.idesc = make_idesc(pair ? kPairBM : kBM, kBN, a.in_dtype == 12 ? 1u : 0u, P.a_mn != 0, P.b_mn != 0);
   const size_t smem = 1024 + P.bar_off + 256;
-  const int grid = static_cast<int>(units1 < num_sms ? units1 : num_sms);
+  const int grid = pair ? 2 * static_cast<int>(units2 < pairs ? units2 : pairs)
+                        : static_cast<int>(units1 < num_sms ? units1 : num_sms);
   void (*kern)(DParams);
   switch (a.out_dtype) {
-    case 0: kern = dense_gemm_kernel<float>; break;
-    case 7: kern = dense_gemm_kernel<__half>; break;
-    case 12: kern = dense_gemm_kernel<__nv_bfloat16>; break;
+    case 0: kern = pair ? dense_gemm_pair_kernel<float> : dense_gemm_kernel<float>; break;
+    case 7: kern = pair ? dense_gemm_pair_kernel<__half> : dense_gemm_kernel<__half>; break;
+    case 12: kern = pair ? dense_gemm_pair_kernel<__nv_bfloat16> : dense_gemm_kernel<__nv_bfloat16>; break;
     default: return cudaErrorInvalidValue;
   }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
