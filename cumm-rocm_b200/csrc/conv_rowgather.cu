@@ -96,6 +96,7 @@ struct KParams {
   int opc;            // offsets packed per chunk (a_row_bytes < 128)
   int upo;            // 16-byte units per packed offset segment
   int stages;
+  int strands;        // strand kernel: pipelines per CTA
   int group_warps;    // gather path: producer warps per chunk
   uint32_t stage_bytes;
   uint32_t b_off;
@@ -956,11 +957,11 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
 // ------------------------------------------------------------------ strand kernel
 // Forward / backward-input over 128-byte (SWIZZLE_128B) or 64-byte
 // (SWIZZLE_64B: C = 64 e4m3, C = 32 bf16 / f16) gathered rows: two CTAs per
-// SM, each one pipeline ("strand") of kSProd producer warps in groups of
-// kSGroupWarps that take the chunks in turn, a ring of P.stages stages (128
-// gathered rows + the weight slab; as many as fit, 4 of 24 KB for 128-byte rows
-// at BN = 64, 8 of 12 KB for 64-byte rows), one MMA warp, a double-buffered TMEM
-// accumulator and four epilogue warps.
+// SM of one or two pipelines ("strands"), which share eight producer warps, the
+// stages (128 gathered rows + the weight slab; 4 of 24 KB for 128-byte rows at
+// BN = 64, 8 of 12 KB for 64-byte rows) and four epilogue warps.  A strand has
+// groups of two producer warps that take its chunks in turn, a ring of stages,
+// one MMA warp and a double-buffered TMEM accumulator.
 //
 // What bounds it, from clock64() counters of every role (200k voxels, C = K =
 // 64): not the tensor core (its warp waits) but the time a chunk holds its
@@ -973,23 +974,28 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
 // without a branch per element 69 / 777 / 33 (with cp.async gathers instead of
 // gather4 67 / 740 / 31); one strand of four stages with warps in groups 61 /
 // 704 / 16; tile ids and masks loaded two tiles ahead 58 / 674 / 16.  Four
-// warps per chunk: 66 / 732 / 19.  Two accumulators per tile for the MMA chain:
-// no change.
+// warps per chunk: 66 / 732 / 19; three of twelve, at 56 registers: 66 / 759 / 16.
+// Two accumulators per tile for the MMA chain: no change.  Two strands of two
+// stages: 54 / 652 / 27 (one strand's chunks go on while the other waits at a
+// tile's end; a lone tile has half the producers), so large calls take two.
 //
 // Tiles are taken in the largest-first order when one is given (strand_tile),
 // else round-robin.  Every role derives its tiles' masks itself (the tile's
 // mask words OR-ed per 32-row group), and the producers read each gather's four
 // indices straight from the sorted index table, so the roles share no index
 // ring.  Needs indices_sorted (16-byte aligned, M % 4 == 0) and BN <= 64.
-constexpr int kStrands = 1;
-constexpr int kSProd = 8;
-constexpr int kSGroupWarps = 2;                       // producer warps per chunk
-constexpr int kSGroups = kSProd / kSGroupWarps;
-constexpr int kSMaxStages = 8;  // stages per strand: 4 of 24 KB (128-byte rows), 8 of 12 KB (64-byte rows)
-constexpr int kSWarps = kEpiWarps + kStrands * (kSProd + 1);  // 13
-constexpr int kSThreads = kSWarps * 32;
-constexpr int kSBars = 2 * kSMaxStages + 7;  // barriers per strand
-constexpr uint32_t kSTmemCols = kStrands * 128;  // per CTA: 2 buffers x BN (<= 64) per strand
+constexpr int kSGroupWarps = 2;  // producer warps per chunk
+// A CTA of NS strands (1 or 2): eight producer warps and four stages of 128-byte
+// rows (24 KB each at BN = 64) or eight of 64-byte rows (12 KB), shared out.
+template <int NS>
+struct Strands {
+  static constexpr int kProd = 8 / NS;  // producer warps of a strand
+  static constexpr int kGroups = kProd / kSGroupWarps;
+  static constexpr int kThreads = (kEpiWarps + NS * (kProd + 1)) * 32;  // 416 or 448
+  static constexpr uint32_t kTmemCols = NS * 128;  // 2 buffers x BN (<= 64) per strand
+  static constexpr int stages(bool wide) { return (wide ? 4 : 8) / NS; }
+};
+constexpr int kSBars = 2 * 8 + 7;  // barriers per strand (eight stages at most)
 
 struct TileMasks {
   uint32_t g[4];    // OR of each 32-row group (unfiltered)
@@ -1042,7 +1048,7 @@ __device__ __forceinline__ int strand_tile(const KParams &P, int pos, int nstr, 
   return P.a.tile_order != nullptr ? static_cast<int>(scheduled_tile(P.a, d)) : d;
 }
 
-template <bool kF8, typename TOut, bool kWide>
+template <bool kF8, typename TOut, bool kWide, int kStrands>
 __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KParams P) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_u32 = smem_u32(smem_raw);
@@ -1050,9 +1056,10 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
   uint8_t *smem = smem_raw + pad;
   const uint32_t smem_base = raw_u32 + pad;
   const ConvRowGatherArgs &A = P.a;
-  // kWide: 128-byte rows (SWIZZLE_128B), four 24 KB stages per strand; else
-  // 64-byte rows (SWIZZLE_64B), eight 12 KB stages
-  constexpr int S = kWide ? 4 : 8;
+  // kWide: 128-byte rows (SWIZZLE_128B); else 64-byte rows (SWIZZLE_64B)
+  using L = Strands<kStrands>;
+  constexpr int kSProd = L::kProd, kSGroups = L::kGroups;
+  constexpr int S = L::stages(kWide);  // at least kSGroups
   constexpr int rb = kWide ? 128 : 64;
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + P.bar_off);
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kStrands * kSBars);
@@ -1080,7 +1087,7 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
     fence_mbar_init();
   }
   if (warp == 0) {
-    tmem_alloc(tmem_slot, kSTmemCols);
+    tmem_alloc(tmem_slot, L::kTmemCols);
     tmem_relinquish();
   }
   // The strand's tiles, two ahead of the one entered: the id of the tile after
@@ -1373,17 +1380,18 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kSTmemCols);
+    tmem_dealloc(tmem_base, L::kTmemCols);
   }
 }
 
 template <bool kF8, typename TOut>
 cudaError_t launch_strands(const KParams &P, int grid, size_t smem, cudaStream_t stream) {
-  void (*kern)(KParams) = P.row_bytes == 128 ? conv_strand_kernel<kF8, TOut, true>
-                                             : conv_strand_kernel<kF8, TOut, false>;
+  const bool wide = P.row_bytes == 128;
+  void (*kern)(KParams) = P.strands == 2 ? (wide ? conv_strand_kernel<kF8, TOut, true, 2> : conv_strand_kernel<kF8, TOut, false, 2>)
+                                         : (wide ? conv_strand_kernel<kF8, TOut, true, 1> : conv_strand_kernel<kF8, TOut, false, 1>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
   if (e != cudaSuccess) return e;
-  kern<<<grid, kSThreads, smem, stream>>>(P);
+  kern<<<grid, P.strands == 2 ? Strands<2>::kThreads : Strands<1>::kThreads, smem, stream>>>(P);
   return cudaGetLastError();
 }
 
@@ -1487,7 +1495,7 @@ cudaError_t launch_conv_rowgather(const ConvRowGatherArgs &a, int num_sms, cudaS
   const uint32_t b_bytes = static_cast<uint32_t>(a.BN) * P.row_bytes;
   P.stage_bytes = a_bytes + b_bytes;
   P.b_off = a_bytes;
-  // Strands (one pipeline per CTA, two CTAs per SM) on the TMA
+  // Strands (one or two pipelines per CTA, two CTAs per SM) on the TMA
   // gather path of 128-byte rows with the sorted index table and BN <= 64
   // (TMEM: 2 buffers x BN columns per CTA); the chunk word of its cursor packs
   // the offset, 11 bits of column block and 15 of column tile, and its tile and
@@ -1495,15 +1503,19 @@ cudaError_t launch_conv_rowgather(const ConvRowGatherArgs &a, int num_sms, cudaS
   if (gather && P.bulk_idx && a.BN <= 64 && !(P.row_bytes == 64 && a.b_mn) && P.cpo < 2048 && a.n_tiles < 32768 &&
       P.num_tiles < (int64_t(1) << 30) && a.a_rows < (int64_t(1) << 31) && a.M < (int64_t(1) << 31) - 1024) {
     if (P.num_tiles == 0) return cudaSuccess;
-    // two CTAs per SM (113 KB each): four stages with 128-byte rows (24 KB at
-    // BN 64), eight with 64-byte rows (12 KB)
-    const int stages = P.row_bytes == 128 ? 4 : 8;
-    P.stages = stages;
-    P.tmem_cols = kSTmemCols;
-    P.bar_off = P.stage_bytes * kStrands * stages;
+    // Two CTAs per SM (113 KB each).  Two strands per CTA where every CTA has
+    // at least three tiles of one column block per offset; kernel us, one
+    // strand / two: 128-byte rows 60k voxels (1.6 tiles) 26 / 30, 80k (2.1) 30 /
+    // 31, 120k (3.2) 41 / 39, 200k 58.4 / 54.4, 300k 79 / 74, 2.6M 674 / 652;
+    // 64-byte rows 40k (1.1) 18 / 25, 80k 28.0 / 26.5, 200k 55 / 48, 300k 76 /
+    // 67.  Two column blocks (C = 128): 60k 41 / 50, 200k 97.9 / 98.2.
+    const int ctas = 2 * num_sms;
+    P.strands = P.cpo == 1 && P.num_tiles >= 3 * static_cast<int64_t>(ctas) ? 2 : 1;
+    P.stages = P.strands == 2 ? Strands<2>::stages(P.row_bytes == 128) : Strands<1>::stages(P.row_bytes == 128);
+    P.tmem_cols = P.strands == 2 ? Strands<2>::kTmemCols : Strands<1>::kTmemCols;
+    P.bar_off = P.stage_bytes * P.strands * P.stages;
     const size_t smem = 1024 + P.bar_off + 512;
-    const int64_t ctas = (P.num_tiles + kStrands - 1) / kStrands;
-    const int grid = static_cast<int>(ctas < 2 * num_sms ? ctas : 2 * num_sms);
+    const int grid = static_cast<int>(P.num_tiles < ctas ? P.num_tiles : ctas);
     {
       const cudaError_t e = prepare_schedule(a, false, stream);
       if (e != cudaSuccess) return e;

@@ -64,3 +64,28 @@ def test_scatter_rows_per_thread(n, c):
     ref = np.ones((2 * n, c))
     ref[inds.cpu().numpy()] += to64(x)
     assert np.array_equal(to64(out), ref)
+
+
+@pytest.mark.parametrize("n", [28284, 28420])
+@pytest.mark.parametrize("C,K", [(64, 256), (32, 256)])
+def test_strands_per_cta(n, C, K):
+    """884 and 892 (row, column) tiles of 64 columns: one strand per CTA below
+    three tiles a CTA, two from there, with a last tile of four rows."""
+    coords = vg.uniform_voxels(n, 48, n)
+    pf, pb, m = po.subm_pairs(coords, (48,) * 3)
+    ms, order = po.sort_by_key_split(m, 0xffffffff)
+    rng = np.random.default_rng(n)
+    bf = torch.bfloat16
+    x = dev(rng.standard_normal((n, C)).astype(np.float32), bf)
+    w = dev(vg.kaiming_uniform(K, 27, C, n), bf)
+    f = find_desp(ConvOpType.kForward, "Tcgen05", tv.bfloat16, tv.bfloat16, tv.bfloat16)
+    out = torch.zeros((n, K), dtype=bf, device="cuda")
+    conv(ConvOpType.kForward, f, x, w, out, pf, ms, order, sorted_indices=True, tile_n=64)
+    assert co.rel_err(to64(out), co.conv_fwd_masked(to64(x), to64(w), pf, ms, order, 128)[0])[0] < 2e-3
+    # the transposed layer's input gradient: rows of C values of dOut, K columns
+    wt = w.permute(2, 1, 0).contiguous()
+    d = find_desp(ConvOpType.kBackwardInput, "Tcgen05", tv.bfloat16, tv.bfloat16, tv.bfloat16)
+    din = torch.zeros((n, K), dtype=bf, device="cuda")
+    conv(ConvOpType.kBackwardInput, d, din, wt, x, pb, ms, order, reverse_mask=True, sorted_indices=True, tile_n=64)
+    ref = co.conv_dgrad_masked(to64(x), to64(wt), pb, ms, order, 128, reverse_mask=True)
+    assert co.rel_err(to64(din), ref)[0] < 2e-3
