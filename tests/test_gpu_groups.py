@@ -3,8 +3,8 @@ scatter's rows per thread, at the sizes where their rules turn: layouts of 1, 2
 and 4 warps a group (several column blocks, packed rows, a dOut ring of two
 buffers), one tile, a ragged last tile and more tiles than CTAs.
 
-Tolerance: bf16 operands with fp32 sums and one bf16 rounding of the result
-(2^-9 a value): norm off by less than 2e-3; fp32 dW: 1e-5 of the terms' norm."""
+Tolerance: bf16 operands with fp32 sums and one bf16 rounding of the result (up
+to 2^-8 a value, about 2^-8 / 2.3 in norm over many): 2e-3 as the other tests; fp32 dW: 1e-5 of the terms' norm."""
 import numpy as np
 import pytest
 import torch
