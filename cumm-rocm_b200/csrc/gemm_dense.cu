@@ -10,7 +10,8 @@
 //
 // B200 design, two kernels: CTA pairs on 256 x 256 tiles where K is long
 // (dense_gemm_pair_kernel; the rule is in launch_dense_gemm), and single CTAs
-// on 128 x 256 tiles.  The single one: persistent CTAs (one per SM) walk
+// on 128 x 256 tiles, or 128 x 128 and 128 x 64 with two CTAs per SM where K
+// is short.  The single one, at 256 columns: persistent CTAs (one per SM) walk
 // (128 x 256 output tile, K split) work units.  Warp 4 loads 128 x 64 A and 256 x 64 B blocks with
 // 2-D TMA boxes into a 4-stage ring (48 KB per stage, SWIZZLE_128B); a
 // row-major operand is K-major for the tensor core and a transposed one is
@@ -31,18 +32,17 @@ namespace scb {
 namespace {
 
 constexpr int kBM = 128, kBN = 256, kBK = 64;
-constexpr int kStages = 4;
+constexpr int kMaxStages = 4;
 constexpr int kThreads = 192;  // warps 0-3 epilogue, 4 TMA producer, 5 MMA issuer
 constexpr int kWarpBuf = 4096;  // bytes per epilogue warp: 32 rows x 128 bytes
 constexpr int kGroupM = 16;    // row tiles per raster group
 constexpr uint32_t kABytes = kBM * kBK * 2;  // 16 KB
-constexpr uint32_t kBBytes = kBN * kBK * 2;  // 32 KB
-constexpr uint32_t kStageBytes = kABytes + kBBytes;
 
 // CTA-pair kernel: a 256 x 256 tile per pair, 128 rows of A and 128 columns of
 // B loaded by each CTA.  Six stages leave room for the epilogue's buffers; seven
 // without them ran 8192^3 in 715 us against 686.
-constexpr int kPairMinBlocks = 16;
+constexpr int kPairMinBlocks = 16;  // K blocks of a unit from which pairs are used
+constexpr int kNarrowBlocks = 8;  // single CTAs: 128 columns up to this many K blocks
 constexpr int kPairBM = 256;
 constexpr int kPairStages = 6;
 constexpr uint32_t kPairBBytes = kBN / 2 * kBK * 2;  // 16 KB
@@ -55,6 +55,8 @@ struct DParams {
   int a_mn, b_mn;  // operand is MN-major (stored transposed relative to the MMA's K-major form)
   int64_t m_tiles, n_tiles, units;
   int splits, kb_per_split, kblocks;
+  int bn, stages;          // single-CTA kernel: columns of a tile, ring stages
+  uint32_t stage_bytes;
   uint32_t bar_off;
   uint32_t idesc;
   float *ws;  // split-K: fp32 [m, n] (ld n), zeroed; else null
@@ -151,16 +153,17 @@ __device__ __forceinline__ void store16(const DParams &P, int64_t row, int64_t c
   }
 }
 
-// Epilogue of one warp's 32 rows (from row0, TMEM address t0) x 256 columns
-// from nb.  Column blocks of 128 bytes go through the warp's 4 KB of shared
-// memory (16-byte units XOR-swizzled by row) so that a store instruction
+// Epilogue of one warp's 32 rows (from row0, TMEM address t0) x the tile's
+// columns from nb.  Column blocks of 128 bytes go through the warp's 4 KB of
+// shared memory (16-byte units XOR-swizzled by row) so that a store instruction
 // writes four whole 128-byte lines; a row per thread wrote 32 pieces of 32
-// lines (16384 x 4096 x 2048: 200 us, staged 187; 8192^3 762 / 750; with K = 256
-// it costs 84 / 86).  Blocks that n cuts, split-K and rows that do not start on
-// 16 bytes are written by the rows' own threads.  With the activation's switch
-// outside the element loop this took 8192 x 8192 x 256 from 367 to 138 us and
-// 304 x 520 x 200 from 48 to 15: a tile's epilogue was longer than its mainloop
-// up to K of about 4096.
+// lines (16384 x 4096 x 2048: 200 us, staged 187; 8192^3 762 / 750), and a
+// block that n cuts went out in single elements (400000 x 32 x 32: 119 us,
+// staged 36; 400000 x 96 x 256: 167 / 63).  Split-K, and rows that do not start
+// or end on 16 bytes, are written by the rows' own threads.  With the
+// activation's switch outside the element loop this took 8192 x 8192 x 256 from
+// 367 to 138 us and 304 x 520 x 200 from 48 to 15: a tile's epilogue was longer
+// than its mainloop up to K of about 4096.
 template <typename TOut>
 __device__ __forceinline__ void store_tile(const DParams &P, uint8_t *buf, int lane, int64_t row0, int64_t nb,
                                            uint32_t t0, bool any) {
@@ -169,13 +172,14 @@ __device__ __forceinline__ void store_tile(const DParams &P, uint8_t *buf, int l
   constexpr int kUnits = 16 * sizeof(TOut) / 16;  // 16-byte units of 16 columns
   const int64_t row = row0 + lane;
   const bool lines = P.ws == nullptr && (reinterpret_cast<uintptr_t>(G.c) & 15u) == 0 &&
-                     (G.ldc * static_cast<int64_t>(sizeof(TOut))) % 16 == 0;
+                     (G.ldc * static_cast<int64_t>(sizeof(TOut))) % 16 == 0 && G.n % (16 / sizeof(TOut)) == 0;
   for (int cb = 0; cb < kBN; cb += kCols) {
-    if (nb + cb >= G.n) break;  // warp-uniform
-    const bool whole = lines && nb + cb + kCols <= G.n;
+    if (nb + cb >= G.n || cb >= P.bn) break;  // warp-uniform
+    const int64_t left = G.n - nb - cb;  // columns from here
 #pragma unroll
     for (int q = 0; q < kCols / 16; ++q) {
       const int64_t col0 = nb + cb + q * 16;
+      if (col0 >= G.n) break;  // warp-uniform
       float acc[16];
       if (any) {
         tmem_ld16(t0 + static_cast<uint32_t>(cb + q * 16), acc);
@@ -183,11 +187,11 @@ __device__ __forceinline__ void store_tile(const DParams &P, uint8_t *buf, int l
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[i] = 0.f;
       }
-      if (!whole) {
-        if (row < G.m && col0 < G.n) store16<TOut>(P, row, col0, acc);
+      if (!lines) {
+        if (row < G.m) store16<TOut>(P, row, col0, acc);
         continue;
       }
-      if (row < G.m) apply16<TOut>(G, row, col0, 16, acc);
+      if (row < G.m) apply16<TOut>(G, row, col0, left - q * 16 < 16 ? left - q * 16 : 16, acc);
 #pragma unroll
       for (int u = 0; u < kUnits; ++u) {
         uint4 w;
@@ -198,21 +202,22 @@ __device__ __forceinline__ void store_tile(const DParams &P, uint8_t *buf, int l
         *reinterpret_cast<uint4 *>(buf + lane * 128 + (((q * kUnits + u) ^ (lane & 7)) << 4)) = w;
       }
     }
-    if (!whole) continue;
+    if (!lines) continue;
     __syncwarp();
-    TOut *dst = static_cast<TOut *>(G.c) + nb + cb + (lane & 7) * (16 / sizeof(TOut));
+    const int unit = (lane & 7) * static_cast<int>(16 / sizeof(TOut));
+    TOut *dst = static_cast<TOut *>(G.c) + nb + cb + unit;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int r = i * 4 + (lane >> 3);
       const uint4 w = *reinterpret_cast<const uint4 *>(buf + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
-      if (row0 + r < G.m) *reinterpret_cast<uint4 *>(dst + (row0 + r) * G.ldc) = w;
+      if (row0 + r < G.m && unit < left) *reinterpret_cast<uint4 *>(dst + (row0 + r) * G.ldc) = w;
     }
     __syncwarp();
   }
 }
 
 template <typename TOut>
-__global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_constant__ DParams P) {
+__global__ void __launch_bounds__(kThreads, 2) dense_gemm_kernel(const __grid_constant__ DParams P) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_u32 = smem_u32(smem_raw);
   const uint32_t pad = (1024u - (raw_u32 & 1023u)) & 1023u;
@@ -222,8 +227,8 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
 
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem + P.bar_off);
   uint64_t *full = bars;
-  uint64_t *empty = bars + kStages;
-  uint64_t *acc_full = empty + kStages;
+  uint64_t *empty = bars + kMaxStages;
+  uint64_t *acc_full = empty + kMaxStages;
   uint64_t *acc_empty = acc_full + 2;
   uint64_t *tile_bar = acc_empty + 2;
   uint64_t *drain_bar = tile_bar + 2;
@@ -235,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kStages; ++i) {
+    for (int i = 0; i < P.stages; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
@@ -249,7 +254,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
     fence_mbar_init();
   }
   if (warp == 5) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(tmem_slot, 2 * P.bn);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -268,7 +273,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
         int64_t mt, nt;
         tile_mn(P, tile, mt, nt);
         const int m0 = static_cast<int>(mt * kBM);
-        const int n0 = static_cast<int>(nt * kBN);
+        const int n0 = static_cast<int>(nt * P.bn);
         const int kb0 = ks * P.kb_per_split;
         const int kb1 = min(P.kblocks, kb0 + P.kb_per_split);
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -277,10 +282,10 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
             ok = false;
             break;
           }
-          const uint32_t sA = smem_base + stage * kStageBytes;
+          const uint32_t sA = smem_base + stage * P.stage_bytes;
           const uint32_t sB = sA + kABytes;
           const int k0 = kb * kBK;
-          mbar_arrive_expect_tx(&full[stage], kStageBytes);
+          mbar_arrive_expect_tx(&full[stage], P.stage_bytes);
           if (P.a_mn) {
             tma_load_2d(sA, &P.ta, m0, k0, &full[stage]);
             tma_load_2d(sA + 8192, &P.ta, m0 + 64, k0, &full[stage]);
@@ -288,12 +293,11 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
             tma_load_2d(sA, &P.ta, k0, m0, &full[stage]);
           }
           if (P.b_mn) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) tma_load_2d(sB + q * 8192, &P.tb, n0 + 64 * q, k0, &full[stage]);
+            for (int q = 0; q < P.bn / 64; ++q) tma_load_2d(sB + q * 8192, &P.tb, n0 + 64 * q, k0, &full[stage]);
           } else {
             tma_load_2d(sB, &P.tb, k0, n0, &full[stage]);
           }
-          if (++stage == kStages) {
+          if (++stage == static_cast<uint32_t>(P.stages)) {
             stage = 0;
             eph ^= 1u;
           }
@@ -325,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
         acc_nkb[ab] = nkb;
         mbar_arrive(&tile_bar[ab]);
         if (!have) break;
-        const uint32_t d = tmem_base + static_cast<uint32_t>(ab * kBN);
+        const uint32_t d = tmem_base + static_cast<uint32_t>(ab * P.bn);
         for (int j = 0; j < nkb; ++j) {
           if (!mbar_wait(&full[stage], fph, abort_flag)) {
             flag_error(G.err, kErrWaitTimeout);
@@ -333,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
             break;
           }
           tc_fence_after();
-          const uint32_t sA = smem_base + stage * kStageBytes;
+          const uint32_t sA = smem_base + stage * P.stage_bytes;
           const uint32_t sB = sA + kABytes;
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
           }
           issued = true;
           mma_commit(&empty[stage]);
-          if (++stage == kStages) {
+          if (++stage == static_cast<uint32_t>(P.stages)) {
             stage = 0;
             fph ^= 1u;
           }
@@ -381,8 +385,8 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
       const int64_t tile = u / P.splits;
       int64_t mt, nt;
       tile_mn(P, tile, mt, nt);
-      store_tile<TOut>(P, smem + kStages * kStageBytes + warp * kWarpBuf, lane, mt * kBM + warp * 32, nt * kBN,
-                       tmem_base + lane_base + static_cast<uint32_t>(ab * kBN), nkb > 0);
+      store_tile<TOut>(P, smem + P.stages * P.stage_bytes + warp * kWarpBuf, lane, mt * kBM + warp * 32, nt * P.bn,
+                       tmem_base + lane_base + static_cast<uint32_t>(ab * P.bn), nkb > 0);
       tc_fence_before();
       mbar_arrive(&acc_empty[ab]);
     }
@@ -392,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, 1) dense_gemm_kernel(const __grid_co
   __syncthreads();
   if (warp == 5) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, 2 * P.bn);
   }
 }
 
@@ -651,22 +655,35 @@ cudaError_t launch_dense_gemm(const GemmArgs &a, float *split_ws, int num_sms, c
   DParams P;
   P.g = a;
   const int splits = dense_gemm_splits(a);
-  const int64_t n_tiles = (a.n + kBN - 1) / kBN;
-  const int64_t units1 = (a.m + kBM - 1) / kBM * n_tiles * splits;
-  const int64_t units2 = (a.m + kPairBM - 1) / kPairBM * n_tiles * splits;
   P.kblocks = static_cast<int>((a.k + kBK - 1) / kBK);
   P.splits = splits;
   P.kb_per_split = P.kblocks > 0 ? (P.kblocks + P.splits - 1) / P.splits : 0;
+  // A short K leaves a tile to its epilogue, so it gets narrow tiles: room for
+  // two CTAs (and epilogues) per SM, and no loads for the padding columns of a
+  // narrow output (1x1x1 convolutions over voxels).  us, 256 columns / narrow:
+  // 400000 x 64 x 64 54 / 35 (64 columns), 400000 x 128 x 128 81 / 54 (128),
+  // 200000 x 64 x 512 84 / 52; outputs wider than the tile (128): 400000 x 256
+  // x 256 136 / 105, 8192 x 8192 x 256 90 / 72, x 512 98 / 86, x 960 111 / 139
+  // (the ring of two stages).  With K of 2048 even 128 columns took 174 us in
+  // narrow tiles against 160 in pairs, so a long K keeps 256.
+  const bool narrow = P.kb_per_split < kPairMinBlocks;
+  P.bn = narrow && a.n <= 64 ? 64 : (narrow && a.n <= 128) || P.kb_per_split <= kNarrowBlocks ? 128 : kBN;
+  const int64_t n_tiles = (a.n + P.bn - 1) / P.bn;
+  const int64_t units1 = (a.m + kBM - 1) / kBM * n_tiles * splits;
+  const int64_t units2 = (a.m + kPairBM - 1) / kPairBM * n_tiles * splits;
+  // A second CTA per SM only where there are tiles for it; else the whole ring.
+  const bool two = P.bn < kBN && units1 > num_sms;
+  P.stages = !two ? kMaxStages : P.bn == 64 ? 3 : 2;
+  P.stage_bytes = kABytes + static_cast<uint32_t>(P.bn) * kBK * 2;
   // CTA pairs where the mainloop is long enough to bound a tile: K >= 1024 per
   // unit.  us, single / pair: 8192 x 8192 x K with K = 512: 90 / 96, 1024:
   // 104 / 104, 1536: 144 / 125, 2048: 188 / 158; 60000 x 512 x K: 51 / 53,
   // 66 / 64, 86 / 76, 107 / 92; 256 x 8192 x K: 16 / 18, 21 / 21, 25 / 23,
-  // 27 / 25.  Below that the epilogue bounds the tile, and the pair's two
-  // epilogues wait for each other.  And only where 256-row tiles take no more
+  // 27 / 25.  Below that the epilogue bounds the tile.  And only where 256-row tiles take no more
   // waves: 1152 x 8192 x 4096 is 288 units in 2 waves of 148, or 160 in 3 waves
   // of 74 (68 / 76); 1280 rows take 3 either way (95 / 79).
   const int pairs = num_sms / 2;
-  const bool pair = P.kb_per_split >= kPairMinBlocks && pairs > 0 &&
+  const bool pair = P.bn == kBN && P.kb_per_split >= kPairMinBlocks && pairs > 0 &&
                     (units2 + pairs - 1) / pairs <= (units1 + num_sms - 1) / num_sms;
   P.a_mn = a.trans_a ? 1 : 0;
   P.b_mn = a.trans_b ? 0 : 1;
@@ -681,17 +698,18 @@ cudaError_t launch_dense_gemm(const GemmArgs &a, float *split_ws, int num_sms, c
                                             static_cast<uint64_t>(a.k > 0 ? a.k : 1),
                                             static_cast<uint64_t>(a.ldb) * 2, 64, 64)
                            : encode_tmap_2d(&P.tb, a.in_dtype, a.b, static_cast<uint64_t>(a.k > 0 ? a.k : 1),
-                                            static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.ldb) * 2, 64, pair ? kBN / 2 : kBN);
+                                            static_cast<uint64_t>(a.n), static_cast<uint64_t>(a.ldb) * 2, 64, pair ? kBN / 2 : P.bn);
   if (!ok_a || !ok_b) return cudaErrorInvalidValue;
   P.m_tiles = pair ? (a.m + kPairBM - 1) / kPairBM : (a.m + kBM - 1) / kBM;
   P.n_tiles = n_tiles;
   P.units = pair ? units2 : units1;
   P.ws = P.splits > 1 ? split_ws : nullptr;
-  P.bar_off = (pair ? kPairStages * kPairStageBytes : kStages * kStageBytes) + 4 * kWarpBuf;
-  P.idesc = make_idesc(pair ? kPairBM : kBM, kBN, a.in_dtype == 12 ? 1u : 0u, P.a_mn != 0, P.b_mn != 0);
+  P.bar_off = (pair ? kPairStages * kPairStageBytes : P.stages * P.stage_bytes) + 4 * kWarpBuf;
+  P.idesc = make_idesc(pair ? kPairBM : kBM, P.bn, a.in_dtype == 12 ? 1u : 0u, P.a_mn != 0, P.b_mn != 0);
   const size_t smem = 1024 + P.bar_off + 256;
+  const int64_t ctas = two ? 2 * num_sms : num_sms;
   const int grid = pair ? 2 * static_cast<int>(units2 < pairs ? units2 : pairs)
-                        : static_cast<int>(units1 < num_sms ? units1 : num_sms);
+                        : static_cast<int>(units1 < ctas ? units1 : ctas);
   void (*kern)(DParams);
   switch (a.out_dtype) {
     case 0: kern = pair ? dense_gemm_pair_kernel<float> : dense_gemm_kernel<float>; break;

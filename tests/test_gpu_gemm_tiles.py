@@ -1,6 +1,6 @@
 """The dense tcgen05 GEMM where its tiles can go wrong: CTA pairs (256 x 256
-tiles, K of at least 1024 per split) and single CTAs (128 x 256), at the edges
-of rows, columns and K, more tiles than CTAs, and every output type through the
+tiles, K of at least 1024 per split) and single CTAs (128 x 256, 128 or 64 by
+the columns), at the edges of rows, columns and K, more tiles than CTAs, and every output type through the
 epilogue's shared-memory lines (whole, cut by n, rows that start off 16 bytes).
 
 Tolerance: an fp32 sum is rounded once per 16 products, at most K / 16 * 2^-23
@@ -26,6 +26,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k,split", [
     (8, 8, 1024, 1), (128, 136, 1024, 1), (264, 512, 1032, 1), (248, 256, 1344, 1), (520, 328, 1096, 1),
     (384, 264, 2176, 2), (256, 256, 1016, 1), (136, 520, 960, 1),
+    (40, 8, 64, 1), (1000, 64, 72, 1), (264, 72, 136, 1), (1000, 128, 960, 1), (300 * 128, 64, 136, 1),
+    (298 * 128 + 8, 96, 200, 1), (200, 120, 520, 2),
 ])
 def test_dense_tile_edges(dt, dc, ta, tb, m, n, k, split):
     rng = np.random.default_rng(m + n + k)
