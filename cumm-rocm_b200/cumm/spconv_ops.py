@@ -80,8 +80,11 @@ class SpconvOps:
         _lib.check(lib.sc_pairs_workspace_size(n, kv, 1, ctypes.byref(need)))
         ws = _ws(need.value, dev)
         sp, ks, dl = _i32x3(spatial_shape), _i32x3(ksize), _i32x3(dilation)
-        # without a split the kernel writes the caller's mask row itself
-        direct = split_masks is None and masks.dtype == torch.int32 and masks[0].is_contiguous()
+        # without a split the kernel writes the caller's mask row itself, where
+        # that is n plain words beside the coordinates (else copy_ converts,
+        # moves or refuses)
+        direct = (split_masks is None and masks.dtype == torch.int32 and masks.device == dev and
+                  tuple(masks[0].shape) == (n,) and masks[0].is_contiguous())
         mask_full = masks[0] if direct else torch.empty(n, dtype=torch.int32, device=dev)
         s = _stream(stream)
         _lib.check(lib.sc_build_subm_pairs(
