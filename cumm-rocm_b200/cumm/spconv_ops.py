@@ -172,10 +172,13 @@ class SpconvOps:
         not read."""
         _lib.require_cuda()
         lib = _lib.load()
-        ind, srt = _t(indices), _t(argsort)
+        ind, srt, msk = _t(indices), _t(argsort), _t(mask)
         kv, n = ind.shape
+        if msk is not None and not (msk.numel() == n and msk.dtype in (torch.int32, torch.uint32) and
+                                    msk.device == ind.device and msk.is_contiguous()):
+            raise ValueError(f"mask must be {n} contiguous 32-bit words on the device of indices")
         out = torch.empty_like(ind)
-        _lib.check(lib.sc_sort_indices_masked(_vp(ind), kv, n, _vp(srt), _vp(_t(mask)), 1 if reverse else 0,
+        _lib.check(lib.sc_sort_indices_masked(_vp(ind), kv, n, _vp(srt), _vp(msk), 1 if reverse else 0,
                                               _vp(out), _stream(stream)))
         if isinstance(indices, tv.Tensor):
             return tv.Tensor(out, tv.int32)

@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from cumm import _lib
+from cumm import tensorview as tv
 from cumm.spconv_ops import SpconvOps
 
 
@@ -65,3 +66,21 @@ def test_subm_mask_elsewhere_or_of_another_form(lib, mask):
     address = _mask_address(lib)
     assert address is not None
     assert mask.device.type == "meta" or address != mask.data_ptr()
+
+
+@pytest.mark.parametrize("mask", [torch.zeros(7, dtype=torch.int32), torch.zeros(9, dtype=torch.int32),
+                                  torch.zeros(8, dtype=torch.int64), torch.zeros(8, dtype=torch.float32),
+                                  torch.zeros(16, dtype=torch.int32)[::2],
+                                  torch.empty(8, dtype=torch.int32, device="meta")])
+def test_sort_indices_refuses_other_masks(lib, mask):
+    """The kernel reads N 32-bit words of the mask."""
+    with pytest.raises(ValueError, match="mask"):
+        SpconvOps.sort_indices(torch.zeros((27, 8), dtype=torch.int32), torch.arange(8, dtype=torch.int32), mask=mask)
+    assert not lib.calls
+
+
+@pytest.mark.parametrize("wrap", [lambda t: t, lambda t: tv.Tensor(t, tv.uint32)])
+def test_sort_indices_takes_a_mask(lib, wrap):
+    mask = torch.zeros(8, dtype=torch.int32)
+    SpconvOps.sort_indices(torch.zeros((27, 8), dtype=torch.int32), torch.arange(8, dtype=torch.int32), mask=wrap(mask))
+    assert lib.calls["sc_sort_indices_masked"][4].value == mask.data_ptr()
