@@ -212,6 +212,11 @@ def _as_i32(v: int) -> int:
     return v - (1 << 32) if v >= (1 << 31) else v
 
 
+def _version(t: torch.Tensor):
+    """Count of torch's writes to t (inference tensors keep none)."""
+    return None if t.is_inference() else t._version
+
+
 @dataclass
 class PairTable:
     """Device-resident pair tables of one sparse conv layer (the inputs of
@@ -234,6 +239,31 @@ class PairTable:
         """P = number of valid (input, output) pairs."""
         return int((self.pairs_fwd >= 0).sum().item())
 
+    def __setattr__(self, name, value):
+        if name in self.__dataclass_fields__:
+            self.__dict__.pop("_built", None)  # see _mark_built
+        object.__setattr__(self, name, value)
+
+    def _mark_built(self):
+        """Notes that the masks name exactly the pairs of the tables, in their
+        argsort's order, as the builder leaves them.  A table or list that is
+        assigned, a mask or argsort that is replaced, and a tensor that is
+        written through torch end that."""
+        rows = self.masks_fwd + self.argsorts_fwd + self.masks_bwd + self.argsorts_bwd
+        self.__dict__["_built"] = (rows, [_version(t) for t in self._tables_and_rows()])
+
+    def _tables_and_rows(self):
+        return [self.pairs_fwd, self.pairs_bwd, *self.masks_fwd, *self.argsorts_fwd, *self.masks_bwd,
+                *self.argsorts_bwd]
+
+    def _masks_exact(self) -> bool:
+        if "_built" not in self.__dict__:
+            return False
+        rows, versions = self.__dict__["_built"]
+        now = self._tables_and_rows()
+        return (len(now) == len(versions) and all(a is b for a, b in zip(now[2:], rows)) and
+                [_version(t) for t in now] == versions)
+
     def sorted_indices(self, which: str = "fwd", split: int = 0) -> torch.Tensor:
         """Index table of `which` ('fwd' or 'bwd') permuted into the argsort
         order the matching convolution uses: forward and backward-weight walk
@@ -243,16 +273,15 @@ class PairTable:
         cache = self.__dict__.setdefault("_sorted_cache", {})
         key = (which, split)
         if key not in cache:
-            # the masks of the rows say which entries exist
-            if which == "fwd":
-                cache[key] = SpconvOps.sort_indices(self.pairs_fwd, self.argsorts_fwd[split],
-                                                    mask=self.masks_fwd[split])
-            elif self.subm:
-                cache[key] = SpconvOps.sort_indices(self.pairs_bwd, self.argsorts_fwd[split],
-                                                    mask=self.masks_fwd[split], reverse=True)
-            else:
-                cache[key] = SpconvOps.sort_indices(self.pairs_bwd, self.argsorts_bwd[split],
-                                                    mask=self.masks_bwd[split])
+            back = self.argsorts_fwd if self.subm else self.argsorts_bwd
+            pairs, order = ((self.pairs_fwd, self.argsorts_fwd) if which == "fwd" else (self.pairs_bwd, back))
+            # the masks that the builder left say which entries exist; others
+            # may disagree with the tables
+            mask = None
+            if self._masks_exact():
+                mask = (self.masks_fwd if which == "fwd" or self.subm else self.masks_bwd)[split]
+            cache[key] = SpconvOps.sort_indices(pairs, order[split], mask=mask,
+                                                reverse=which != "fwd" and self.subm)
         return cache[key]
 
     def tile_order(self, which: str = "fwd", split: int = 0) -> torch.Tensor:
@@ -304,11 +333,15 @@ def build_pair_table(coords: torch.Tensor, spatial_shape: Sequence[int], ksize=(
         SpconvOps.generate_subm_conv_inds(coords, pairs, m, spatial_shape, ksize, dilation,
                                           stream=stream)
         masks, sorts = _sorted_masks(m[0], splits, kv, stream)
-        return PairTable(n, n, kv, True, pairs[0], pairs[1], masks, sorts, split_masks=splits,
-                         out_inds=coords, out_spatial=list(spatial_shape))
+        pt = PairTable(n, n, kv, True, pairs[0], pairs[1], masks, sorts, split_masks=splits,
+                       out_inds=coords, out_spatial=list(spatial_shape))
+        pt._mark_built()
+        return pt
     out_inds, pf, pb, mf, mb, out_sp = SpconvOps.generate_conv_inds(
         coords, batch_size, spatial_shape, ksize, stride, padding, dilation, stream)
     masks, sorts = _sorted_masks(mf, splits, kv, stream)
     masks_b, sorts_b = _sorted_masks(mb, splits, kv, stream)
-    return PairTable(n, out_inds.shape[0], kv, False, pf, pb, masks, sorts, masks_b, sorts_b,
-                     splits, out_inds, out_sp)
+    pt = PairTable(n, out_inds.shape[0], kv, False, pf, pb, masks, sorts, masks_b, sorts_b,
+                   splits, out_inds, out_sp)
+    pt._mark_built()
+    return pt

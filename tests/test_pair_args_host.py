@@ -1,11 +1,13 @@
 """Host side of the pair builder's calls, with the native library replaced by a
 recorder: which addresses a call hands over, and what it refuses before that."""
+import dataclasses
+
 import pytest
 import torch
 
 from cumm import _lib
 from cumm import tensorview as tv
-from cumm.spconv_ops import SpconvOps
+from cumm.spconv_ops import PairTable, SpconvOps, build_pair_table
 
 
 class Recorder:
@@ -84,3 +86,36 @@ def test_sort_indices_takes_a_mask(lib, wrap):
     mask = torch.zeros(8, dtype=torch.int32)
     SpconvOps.sort_indices(torch.zeros((27, 8), dtype=torch.int32), torch.arange(8, dtype=torch.int32), mask=wrap(mask))
     assert lib.calls["sc_sort_indices_masked"][4].value == mask.data_ptr()
+
+
+def _table(n=8, **kw):
+    row = lambda: torch.arange(n, dtype=torch.int32)
+    pairs = lambda: torch.zeros((27, n), dtype=torch.int32)
+    return PairTable(n, n, 27, False, pairs(), pairs(), [row()], [row()], **kw)
+
+
+def _sorted_with(lib, pt, which):
+    lib.calls.clear()
+    pt.sorted_indices(which)
+    mask = lib.calls["sc_sort_indices_masked"][4]
+    return None if mask is None else mask.value
+
+
+def test_tables_made_by_the_caller_are_sorted_whole(lib):
+    """Masks that did not come with the tables may name fewer pairs than these
+    hold (rows of one split, merged words) or be absent: every entry is read."""
+    assert _sorted_with(lib, _table(), "fwd") is None
+    pt = _table(argsorts_bwd=[torch.arange(8, dtype=torch.int32)])
+    assert _sorted_with(lib, pt, "bwd") is None
+
+
+@pytest.mark.parametrize("change", [lambda m: m[0].bitwise_and_(1), lambda m: m.__setitem__(0, m[0] & 1)])
+def test_built_tables_are_sorted_by_their_own_masks(lib, change):
+    coords = torch.zeros((8, 4), dtype=torch.int32)
+    pt = build_pair_table(coords, (4, 4, 4))
+    assert _sorted_with(lib, pt, "bwd") == pt.masks_fwd[0].data_ptr()
+    change(pt.masks_fwd)
+    assert _sorted_with(lib, pt, "fwd") is None
+    # a copy with other masks is a table made by the caller
+    pt = build_pair_table(coords, (4, 4, 4))
+    assert _sorted_with(lib, dataclasses.replace(pt, masks_fwd=[pt.masks_fwd[0] & 1]), "fwd") is None
