@@ -38,9 +38,12 @@ _I32x3 = ctypes.c_int32 * 3
 
 
 def _i32x3(v: Sequence[int]):
-    """Three ints as a host array (an argument of the C entry points)."""
-    a, b, c = v
-    return _I32x3(int(a), int(b), int(c))
+    """The first three ints as a host array (an argument of the C entry
+    points).  ctypes would wrap a value that 32 bits do not hold."""
+    a, b, c = (int(x) for x in list(v)[:3])
+    if not all(-(1 << 31) <= x < 1 << 31 for x in (a, b, c)):
+        raise ValueError(f"{a}, {b}, {c}: a value does not fit 32 bits")
+    return _I32x3(a, b, c)
 
 
 def _stream(stream: int):

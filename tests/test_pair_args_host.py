@@ -2,6 +2,7 @@
 recorder: which addresses a call hands over, and what it refuses before that."""
 import dataclasses
 
+import numpy as np
 import pytest
 import torch
 
@@ -119,3 +120,21 @@ def test_built_tables_are_sorted_by_their_own_masks(lib, change):
     # a copy with other masks is a table made by the caller
     pt = build_pair_table(coords, (4, 4, 4))
     assert _sorted_with(lib, dataclasses.replace(pt, masks_fwd=[pt.masks_fwd[0] & 1]), "fwd") is None
+
+
+@pytest.mark.parametrize("v", [(2 ** 31, 4, 4), (4, 2 ** 32 + 4, 4), (4, 4, -2 ** 31 - 1), (4, 4)])
+def test_sizes_outside_int32_are_refused(lib, v):
+    """A size that 32 bits do not hold is an error and not another size."""
+    coords = torch.zeros((8, 4), dtype=torch.int32)
+    with pytest.raises((RuntimeError, ValueError)):
+        build_pair_table(coords, v)
+    with pytest.raises((RuntimeError, ValueError)):
+        build_pair_table(coords, v, subm=False)
+    assert not {"sc_build_subm_pairs", "sc_build_conv_outputs"} & set(lib.calls)
+
+
+def test_sizes_of_any_integer_kind(lib):
+    coords = torch.zeros((8, 4), dtype=torch.int32)
+    for v in (torch.tensor([4, 5, 6]), np.array([4, 5, 6]), (4.0, 5, 6), (4, 5, 6, 7)):
+        build_pair_table(coords, v)
+        assert list(lib.calls["sc_build_subm_pairs"][2])[:3] == [4, 5, 6]
