@@ -778,6 +778,8 @@ constexpr int kMaskBins = 256;
 constexpr int kMaskPasses = 4;
 // Up to this many tiles a tile sums the counts before it itself (one short row per digit).
 constexpr int kMaskRowTiles = 256;
+// Up to this many rows tiles have 1024 of them, above 2048.
+constexpr int64_t kMaskSmallRows = (int64_t(kMaskRowTiles) << 10) / 2;
 
 struct MaskSort {
   int64_t n;
@@ -962,7 +964,7 @@ MaskSort mask_sort_plan(int64_t n, uint32_t split) {
   // Small tiles while that keeps the count rows short: more blocks, fewer
   // serial rounds per warp, against more rows for every tile to sum (200k rows
   // a pass: 11.3 us with 196 tiles, 10.1 with 98).
-  P.tile_shift = n <= (int64_t(kMaskRowTiles) << 10) / 2 ? 10 : 11;
+  P.tile_shift = n <= kMaskSmallRows ? 10 : 11;
   P.tiles = static_cast<int>((n + (int64_t(1) << P.tile_shift) - 1) >> P.tile_shift);
   P.pitch = (P.tiles + 3) & ~3;
   return P;
@@ -1267,9 +1269,17 @@ cudaError_t sort_indices(const int32_t *indices, int kv, int64_t n, const int32_
   return cudaGetLastError();
 }
 
+// Never less for more rows (a workspace is often sized once, for the largest
+// call): just above kMaskSmallRows there are fewer tiles, so the counts of the
+// small tiles are what is asked for.
 int64_t sort_workspace_bytes(int64_t n) {
-  const MaskSort P = mask_sort_plan(n, 0xffffffffu);
-  return 3 * align_up(n * 4) + align_up((static_cast<int64_t>(P.pitch) + 1) * kMaskPasses * kMaskBins * 4) + 256;
+  if (n <= 0) return 0;
+  int64_t pitch = mask_sort_plan(n, 0xffffffffu).pitch;
+  if (n > kMaskSmallRows) {
+    const int64_t small = mask_sort_plan(kMaskSmallRows, 0xffffffffu).pitch;
+    pitch = pitch > small ? pitch : small;
+  }
+  return 3 * align_up(n * 4) + align_up((pitch + 1) * kMaskPasses * kMaskBins * 4) + 256;
 }
 
 cudaError_t sort_masks_split(uint32_t *data, int64_t n, uint32_t split_mask, int32_t *argsort,
