@@ -27,6 +27,7 @@
 #include <cuda.h>
 
 #include "kernels.h"
+#include "launch_rules.h"
 
 namespace scb {
 namespace {
@@ -941,11 +942,9 @@ cudaError_t launch_conv_wgrad(const ConvWgradArgs &a, int num_sms, cudaStream_t 
   per_group = (P.n_mtiles + n_groups - 1) / n_groups;
   P.tiles_per_group = per_group;
   P.n_groups = (P.n_mtiles + per_group - 1) / per_group;
-  // row splits: the caller's split_k_slices, else as many CTAs as run at once
-  // (one per SM, two in the pair layout): rounding the splits up left a second
-  // wave of a few CTAs (60k voxels, C = K = 128: 7 groups x 22 splits on 148 SMs)
-  const int ctas = (pair ? 2 : 1) * num_sms;
-  int splits = a.split_k > 0 ? a.split_k : ctas > P.n_groups ? ctas / P.n_groups : 1;
+  // row splits: the caller's split_k_slices, else wgrad_row_splits' for the
+  // CTAs that run at once (one per SM, two in the pair layout)
+  int splits = a.split_k > 0 ? a.split_k : wgrad_row_splits(P.n_chunks, P.n_groups, (pair ? 2 : 1) * num_sms);
   if (splits > P.n_chunks) splits = P.n_chunks;
   P.chunks_per_cta = (P.n_chunks + splits - 1) / splits;
   splits = (P.n_chunks + P.chunks_per_cta - 1) / P.chunks_per_cta;

@@ -34,7 +34,7 @@ class FwdConfig:
 
 @dataclass(frozen=True)
 class WgradConfig:
-    split_k: int = 0     # row splits of the backward-weight kernel; 0: about one CTA per SM
+    split_k: int = 0     # row splits of the backward-weight kernel; 0: the launcher's rule
 
     def __str__(self):
         return f"splitk{self.split_k or 'auto'}"

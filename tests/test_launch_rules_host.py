@@ -1,0 +1,41 @@
+"""The launchers' rules on the CPU (csrc/launch_rules.h compiled by itself)."""
+import ctypes
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "cumm-rocm_b200" / "csrc"
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    if shutil.which("g++") is None:
+        pytest.skip("no host compiler")
+    d = tmp_path_factory.mktemp("rules")
+    (d / "rules.cpp").write_text('#include "launch_rules.h"\n'
+                                 'extern "C" int wgrad(int chunks, int groups, int ctas) '
+                                 '{ return scb::wgrad_row_splits(chunks, groups, ctas); }\n')
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", str(CSRC), str(d / "rules.cpp"), "-o",
+                    str(d / "rules.so")], check=True)
+    return ctypes.CDLL(str(d / "rules.so"))
+
+
+@pytest.mark.parametrize("ctas", [148, 296, 132, 7])
+def test_wgrad_chain_never_longer_than_with_filled_ctas(rules, ctas):
+    """A split's chunks are one chain of additions: its length bounds dW's
+    error, so rounding the splits must not lengthen it; and the splits leave no
+    wave of fewer CTAs than the rounded-up ones would."""
+    for groups in list(range(1, 60)) + [108, 147, 148, 149, 200, 296, 297, 700]:
+        for chunks in (1, 2, 3, 7, 30, 79, 157, 313, 625, 938, 3125, 40625):
+            s = rules.wgrad(chunks, groups, ctas)
+            assert 1 <= s <= chunks
+            filled = min(-(-ctas // groups), chunks)
+            chain = -(-chunks // s)
+            assert chain <= -(-chunks // filled), (groups, chunks)
+            assert -(-chunks // chain) == s  # no empty split
+            waves = lambda n: -(-n * groups // ctas)
+            full = -(-chunks // -(-chunks // filled))
+            assert waves(s) <= max(waves(full), 2), (groups, chunks)
+            assert waves(s) * chain <= waves(full) * -(-chunks // filled), (groups, chunks)
