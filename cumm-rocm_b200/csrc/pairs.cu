@@ -246,13 +246,17 @@ subm_pairs_kernel(const int32_t *coords, int vec, int64_t n, Geom g, GroupTable 
     const bool want_side = (q == 0 || q == 3) && gx + side >= 0 && gx + side < ng;
     const unsigned long long key0 = static_cast<unsigned long long>(lin_key(co.x, z, y, gx, gsp));
     // where the lane beside holds the neighbour group (rows in scan order), its
-    // nine probes are this lane's too
+    // nine probes are this lane's too; both in the grid, as a voxel outside it
+    // has the linear key of a group of another row
     const int lane = threadIdx.x & 31;
+    const bool inside = live && co.x >= 0 && z >= 0 && y >= 0 && x >= 0 && z < g.spatial[0] && y < g.spatial[1] &&
+                        x < g.spatial[2];
     const unsigned long long key_up = __shfl_up_sync(0xffffffffu, key0, 1);
     const unsigned long long key_dn = __shfl_down_sync(0xffffffffu, key0, 1);
-    const unsigned alive = __ballot_sync(0xffffffffu, live);
-    const bool shared = want_side && (q == 0 ? lane > 0 && key_up == key0 - 1
-                                             : lane < 31 && ((alive >> (lane + 1)) & 1u) && key_dn == key0 + 1);
+    const unsigned in_grid = __ballot_sync(0xffffffffu, inside);
+    const int beside = (lane + side) & 31;
+    const bool shared = inside && want_side && lane + side == beside && ((in_grid >> beside) & 1u) &&
+                        (q == 0 ? key_up == key0 - 1 : key_dn == key0 + 1);
     const bool has_side = live && want_side && !shared;
     const long long dz = static_cast<long long>(g.spatial[1]) * ng;
     __shared__ int sj[27][128];  // [offset][thread]

@@ -1,0 +1,39 @@
+"""Submanifold pairs where the lookups' short cuts end: rows beside a voxel
+outside the grid, whose linear key is that of another row's group."""
+import numpy as np
+import pytest
+import torch
+
+from cumm import _lib
+from cumm.spconv_ops import build_pair_table
+
+pytestmark = pytest.mark.gpu
+
+
+def _neighbours(c, spatial):
+    """pairs_fwd by the definition: the voxel of the grid at coord + offset - 1."""
+    at = {tuple(v): i for i, v in reversed(list(enumerate(c.tolist()))) if all(0 <= v[d + 1] < spatial[d] for d in range(3))}
+    out = np.full((27, len(c)), -1, np.int32)
+    for i, (b, z, y, x) in enumerate(c.tolist()):
+        for k in range(27):
+            out[k, i] = at.get((b, z + k // 9 - 1, y + k // 3 % 3 - 1, x + k % 3 - 1), -1)
+    return out
+
+
+@pytest.mark.parametrize("outside", [(0, 1, 1, 8), (0, 1, 1, 9), (0, 0, 6, 0), (0, 0, 5, 8), (0, 2, -2, 0), (0, 1, 3, -3),
+                                     (-1, 7, 2, 3)])
+@pytest.mark.parametrize("first", [True, False])
+def test_rows_beside_a_voxel_outside_the_grid(outside, first):
+    """Every voxel of a 4 x 4 x 8 grid once, in scan order, with a voxel outside
+    the grid before or after each row: the voxels of the grid keep their
+    neighbours, and the call leaves its error bit."""
+    spatial = (4, 4, 8)
+    c = np.stack(np.meshgrid([0], range(4), range(4), range(8), indexing="ij"), -1).reshape(-1, 4).astype(np.int32)
+    for at in range(0, len(c) + 1):
+        rows = np.insert(c, at, outside, axis=0)
+        if not first:
+            rows = rows[::-1].copy()
+        pt = build_pair_table(torch.from_numpy(rows).cuda(), spatial)
+        assert _lib.device_error_bits() == 1
+        inside = np.delete(np.arange(len(rows)), at if first else len(c) - at)
+        assert np.array_equal(pt.pairs_fwd.cpu().numpy()[:, inside], _neighbours(rows, spatial)[:, inside]), at
