@@ -28,6 +28,7 @@ namespace {
 constexpr int kSlice = 32;           // reduction elements per stage
 constexpr int kPitch = kSlice + 4;   // floats between rows of a [row][slice] tile: 16-byte aligned, conflict-free
 constexpr int kStages = 3;
+constexpr int kMaxGridYZ = 65535;    // more blocks along y or z take several launches
 
 __device__ __forceinline__ uint32_t smem_addr(const float *p) { return smem_u32(p); }
 
@@ -47,7 +48,7 @@ __device__ __forceinline__ void copy4(float *dst, const float *src, const float 
 // reduction elements, in ascending order.
 template <bool kFwd, bool kVec, int kRows, int kCols>
 __global__ void __launch_bounds__(kRows * 2)
-simt_fwd_kernel(const ConvSimtArgs A, int n_red, int n_out) {
+simt_fwd_kernel(const ConvSimtArgs A, int n_red, int n_out, int col_block0) {
   constexpr int kThreads = kRows * 2;
   constexpr int kPer = kCols / 8;
   constexpr int kATile = kRows * kPitch;
@@ -61,7 +62,7 @@ simt_fwd_kernel(const ConvSimtArgs A, int n_red, int n_out) {
   __shared__ int s_k[32];
   const int tid = threadIdx.x;
   const int64_t row0 = static_cast<int64_t>(blockIdx.x) * kRows;
-  const int nb = blockIdx.y * kCols;
+  const int nb = (col_block0 + static_cast<int>(blockIdx.y)) * kCols;
   if (tid == 0) s_km = 0;
   __syncthreads();
   // the mask tile may be wider than the block's rows
@@ -83,7 +84,7 @@ simt_fwd_kernel(const ConvSimtArgs A, int n_red, int n_out) {
   }
   __syncthreads();
   uint32_t km = s_km & A.mask_filter;
-  if (kFwd && A.mask_out != nullptr && tid == 0 && blockIdx.y == 0 && row0 == mask0)
+  if (kFwd && A.mask_out != nullptr && tid == 0 && nb == 0 && row0 == mask0)
     A.mask_out[row0 / A.tile_m_desp] = km;
   if (!kFwd && km == 0) return;  // dgrad early exit (kernel.py:875-882)
   if (!kFwd && A.reverse) km = __brev(km) >> (32 - A.kv);
@@ -230,7 +231,7 @@ constexpr int kWRange = 1024;        // most rows per block (at most 32 chunks)
 
 template <bool kVec>
 __global__ void __launch_bounds__(kWThreads)
-simt_wgrad_kernel(const ConvSimtArgs A, int rows_per_block, int vec_out) {
+simt_wgrad_kernel(const ConvSimtArgs A, int rows_per_block, int vec_out, int64_t row_block0) {
   extern __shared__ __align__(16) float sm[];  // [kStages][2][kWChunk][32]
   __shared__ int s_sig[kWRange], s_idx[kWRange];
   __shared__ unsigned s_some;
@@ -238,7 +239,7 @@ simt_wgrad_kernel(const ConvSimtArgs A, int rows_per_block, int vec_out) {
   const int ncb = (A.C + 31) / 32;
   const int n0 = (blockIdx.y / ncb) * 32;
   const int c0 = (blockIdx.y % ncb) * 32;
-  const int64_t r0 = static_cast<int64_t>(blockIdx.z) * rows_per_block;
+  const int64_t r0 = (row_block0 + blockIdx.z) * rows_per_block;
   const int rows = static_cast<int>(min(static_cast<int64_t>(rows_per_block), A.M - r0));
   const int tid = threadIdx.x;
   if (!((A.mask_filter >> k) & 1u)) return;
@@ -362,9 +363,14 @@ cudaError_t launch_fwd(const ConvSimtArgs &a, int n_red, int n_out, cudaStream_t
   auto kern = simt_fwd_kernel<kFwd, kVec, kRows, kCols>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  const dim3 grid(static_cast<unsigned>((a.M + kRows - 1) / kRows), (n_out + kCols - 1) / kCols);
-  kern<<<grid, kRows * 2, smem, stream>>>(a, n_red, n_out);
-  return cudaGetLastError();
+  const int cols = (n_out - 1) / kCols + 1;
+  for (int c0 = 0; c0 < cols; c0 += kMaxGridYZ) {
+    const dim3 grid(static_cast<unsigned>((a.M + kRows - 1) / kRows), cols - c0 < kMaxGridYZ ? cols - c0 : kMaxGridYZ);
+    kern<<<grid, kRows * 2, smem, stream>>>(a, n_red, n_out, c0);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 template <bool kFwd, bool kVec>
@@ -391,15 +397,21 @@ cudaError_t launch_conv_simt(const ConvSimtArgs &a, cudaStream_t stream) {
     rows = (rows + kWChunk - 1) / kWChunk * kWChunk;
     if (rows < 4 * kWChunk) rows = 4 * kWChunk;
     if (rows > kWRange) rows = kWRange;
-    const dim3 grid(a.kv, ((a.K + 31) / 32) * ((a.C + 31) / 32), static_cast<unsigned>((a.M + rows - 1) / rows));
     const bool v = vec && a.K % 4 == 0 && a.C % 4 == 0;
     const int vec_out = a.C % 4 == 0 && aligned16(a.out);
     auto kern = v ? simt_wgrad_kernel<true> : simt_wgrad_kernel<false>;
     const int smem = kStages * 2 * kWChunk * 32 * static_cast<int>(sizeof(float));
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kWThreads, smem, stream>>>(a, static_cast<int>(rows), vec_out);
-    return cudaGetLastError();
+    const int64_t blocks = (a.M + rows - 1) / rows;
+    for (int64_t z0 = 0; z0 < blocks; z0 += kMaxGridYZ) {
+      const dim3 grid(a.kv, ((a.K + 31) / 32) * ((a.C + 31) / 32),
+                      static_cast<unsigned>(blocks - z0 < kMaxGridYZ ? blocks - z0 : kMaxGridYZ));
+      kern<<<grid, kWThreads, smem, stream>>>(a, static_cast<int>(rows), vec_out, z0);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
   }
   const int n_red = a.op == 0 ? a.C : a.K;
   const int n_out = a.op == 0 ? a.K : a.C;
