@@ -388,7 +388,7 @@ int sc_conv_implicit_gemm(const sc_conv_params *p) {
       e = cudaMemsetAsync(p->workspace, 0, p->K * p->kv * p->C * 4, s);
       if (e != cudaSuccess) return cuda_fail(e, "zero workspace");
     }
-    e = scb::launch_conv_simt(a, s);
+    e = scb::launch_conv_simt(a, sms, s);
     if (e != cudaSuccess) return cuda_fail(e, "conv_simt launch");
     if (op == SC_CONV_BACKWARD_WEIGHT) {
       scb::EpiParams ep{};

@@ -21,6 +21,7 @@
 // 453 -> 59 us, backward-input 449 -> 58, backward-weight 433 -> 42.
 // A 16 x 1 register tile (one address per warp and A read) was slower: 67 us.
 #include "kernels.h"
+#include "launch_rules.h"
 
 namespace scb {
 namespace {
@@ -227,7 +228,7 @@ simt_fwd_kernel(const ConvSimtArgs A, int n_red, int n_out, int col_block0) {
 // thread); their partial tiles are added with v4 reductions.
 constexpr int kWThreads = 128;
 constexpr int kWChunk = 64;          // rows per stage
-constexpr int kWRange = 1024;        // most rows per block (at most 32 chunks)
+constexpr int kWRange = 1024;        // most rows per block: 16 chunks, a bit each in s_some
 
 template <bool kVec>
 __global__ void __launch_bounds__(kWThreads)
@@ -374,10 +375,10 @@ cudaError_t launch_fwd(const ConvSimtArgs &a, int n_red, int n_out, cudaStream_t
 }
 
 template <bool kFwd, bool kVec>
-cudaError_t pick_fwd(const ConvSimtArgs &a, int n_red, int n_out, cudaStream_t stream) {
+cudaError_t pick_fwd(const ConvSimtArgs &a, int n_red, int n_out, int num_sms, cudaStream_t stream) {
   // 64 rows a block where the mask tile has them; 64 columns (half the reads
   // of A per product) where they exist and the rows alone fill the GPU
-  const bool wide = n_out > 32 && a.M >= 64 * 296;
+  const bool wide = simt_wide_columns(a.M, n_out, num_sms);
   if (a.tile_m_desp == 32)
     return wide ? launch_fwd<kFwd, kVec, 32, 64>(a, n_red, n_out, stream)
                 : launch_fwd<kFwd, kVec, 32, 32>(a, n_red, n_out, stream);
@@ -387,16 +388,11 @@ cudaError_t pick_fwd(const ConvSimtArgs &a, int n_red, int n_out, cudaStream_t s
 
 }  // namespace
 
-cudaError_t launch_conv_simt(const ConvSimtArgs &a, cudaStream_t stream) {
+cudaError_t launch_conv_simt(const ConvSimtArgs &a, int num_sms, cudaStream_t stream) {
   if (a.M == 0) return cudaSuccess;
   const bool vec = aligned16(a.a) && aligned16(a.b);
   if (a.op == 2) {
-    // about six blocks per SM, in whole chunks of rows
-    const int tiles = a.kv * ((a.K + 31) / 32) * ((a.C + 31) / 32);
-    int64_t rows = (a.M * tiles + 148 * 6 - 1) / (148 * 6);
-    rows = (rows + kWChunk - 1) / kWChunk * kWChunk;
-    if (rows < 4 * kWChunk) rows = 4 * kWChunk;
-    if (rows > kWRange) rows = kWRange;
+    const int64_t rows = simt_wgrad_rows(a.M, a.kv * ((a.K + 31) / 32) * ((a.C + 31) / 32), num_sms, kWChunk, kWRange);
     const bool v = vec && a.K % 4 == 0 && a.C % 4 == 0;
     const int vec_out = a.C % 4 == 0 && aligned16(a.out);
     auto kern = v ? simt_wgrad_kernel<true> : simt_wgrad_kernel<false>;
@@ -416,8 +412,8 @@ cudaError_t launch_conv_simt(const ConvSimtArgs &a, cudaStream_t stream) {
   const int n_red = a.op == 0 ? a.C : a.K;
   const int n_out = a.op == 0 ? a.K : a.C;
   const bool v = vec && n_red % 4 == 0 && (a.op == 0 || n_out % 4 == 0);
-  if (a.op == 0) return v ? pick_fwd<true, true>(a, n_red, n_out, stream) : pick_fwd<true, false>(a, n_red, n_out, stream);
-  return v ? pick_fwd<false, true>(a, n_red, n_out, stream) : pick_fwd<false, false>(a, n_red, n_out, stream);
+  if (a.op == 0) return v ? pick_fwd<true, true>(a, n_red, n_out, num_sms, stream) : pick_fwd<true, false>(a, n_red, n_out, num_sms, stream);
+  return v ? pick_fwd<false, true>(a, n_red, n_out, num_sms, stream) : pick_fwd<false, false>(a, n_red, n_out, num_sms, stream);
 }
 
 }  // namespace scb

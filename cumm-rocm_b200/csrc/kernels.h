@@ -145,7 +145,7 @@ struct ConvSimtArgs {
   EpiParams epi;
   int *err;
 };
-cudaError_t launch_conv_simt(const ConvSimtArgs &a, cudaStream_t stream);
+cudaError_t launch_conv_simt(const ConvSimtArgs &a, int num_sms, cudaStream_t stream);
 
 // ------------------------------------------------------------------ GEMM
 struct GemmArgs {

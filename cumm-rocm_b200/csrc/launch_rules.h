@@ -26,4 +26,17 @@ inline int wgrad_row_splits(int chunks, int groups, int ctas) {
   return two > filled ? clamp(two) : one;
 }
 
+// fp32 forward / backward-input: 64 output columns a block instead of 32 where
+// the 64-row blocks alone are two per SM.
+inline bool simt_wide_columns(long long rows, int columns, int sms) { return columns > 32 && rows >= 64ll * 2 * sms; }
+
+// fp32 backward-weight: rows per block, in whole chunks, for about six blocks
+// per SM; at least four chunks, at most `range` rows.
+inline long long simt_wgrad_rows(long long rows, int tiles, int sms, int chunk, int range) {
+  long long r = (rows * tiles + sms * 6 - 1) / (sms * 6);
+  r = (r + chunk - 1) / chunk * chunk;
+  if (r < 4 * chunk) r = 4 * chunk;
+  return r > range ? range : r;
+}
+
 }  // namespace scb

@@ -16,10 +16,17 @@ def rules(tmp_path_factory):
     d = tmp_path_factory.mktemp("rules")
     (d / "rules.cpp").write_text('#include "launch_rules.h"\n'
                                  'extern "C" int wgrad(int chunks, int groups, int ctas) '
-                                 '{ return scb::wgrad_row_splits(chunks, groups, ctas); }\n')
+                                 '{ return scb::wgrad_row_splits(chunks, groups, ctas); }\n'
+                                 'extern "C" int wide(long long rows, int columns, int sms) '
+                                 '{ return scb::simt_wide_columns(rows, columns, sms); }\n'
+                                 'extern "C" long long simt_rows(long long rows, int tiles, int sms) '
+                                 '{ return scb::simt_wgrad_rows(rows, tiles, sms, 64, 1024); }\n')
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", str(CSRC), str(d / "rules.cpp"), "-o",
                     str(d / "rules.so")], check=True)
-    return ctypes.CDLL(str(d / "rules.so"))
+    lib = ctypes.CDLL(str(d / "rules.so"))
+    lib.wide.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
+    lib.simt_rows.argtypes, lib.simt_rows.restype = lib.wide.argtypes, ctypes.c_longlong
+    return lib
 
 
 @pytest.mark.parametrize("ctas", [148, 296, 132, 7])
@@ -39,3 +46,18 @@ def test_wgrad_chain_never_longer_than_with_filled_ctas(rules, ctas):
             full = -(-chunks // -(-chunks // filled))
             assert waves(s) <= max(waves(full), 2), (groups, chunks)
             assert waves(s) * chain <= waves(full) * -(-chunks // filled), (groups, chunks)
+
+
+@pytest.mark.parametrize("sms", [148, 132, 20])
+def test_simt_rules_follow_the_sm_count(rules, sms):
+    """64 columns from two 64-row blocks per SM; about six row ranges' blocks
+    per SM between the least and the most rows of a block."""
+    assert rules.wide(128 * sms, 33, sms) and not rules.wide(128 * sms - 1, 33, sms)
+    assert not rules.wide(128 * sms, 32, sms)
+    for tiles in (1, 27, 108):
+        for rows in (1, 1000, 20000, 300000, 70000000):
+            r = rules.simt_rows(rows, tiles, sms)
+            assert r % 64 == 0 and 256 <= r <= 1024
+            blocks = -(-rows // r) * tiles
+            assert r == 256 or blocks >= 3 * sms
+            assert r == 1024 or blocks <= 6 * sms + tiles
