@@ -1,11 +1,13 @@
 """Submanifold pairs where the lookups' short cuts end: rows beside a voxel
-outside the grid, whose linear key is that of another row's group."""
+outside the grid, whose linear key is that of another row's group, and buckets
+of the group table that overflow."""
 import numpy as np
 import pytest
 import torch
 
 from cumm import _lib
 from cumm.spconv_ops import build_pair_table
+from oracle import pairs_oracle as po
 
 pytestmark = pytest.mark.gpu
 
@@ -37,3 +39,28 @@ def test_rows_beside_a_voxel_outside_the_grid(outside, first):
         assert _lib.device_error_bits() == 1
         inside = np.delete(np.arange(len(rows)), at if first else len(c) - at)
         assert np.array_equal(pt.pairs_fwd.cpu().numpy()[:, inside], _neighbours(rows, spatial)[:, inside]), at
+
+
+def _bucket(key, log2cap):
+    """The hash of pairs.cu's group table: the bucket of eight slots of a key."""
+    m = np.uint64(0xffffffff)
+    h = (key & m) + (((key >> np.uint64(32)) * np.uint64(0x85ebca6b)) & m) & m
+    h = h * np.uint64(0x9e3779b1) & m
+    h ^= h >> np.uint64(15)
+    h = h * np.uint64(0x2c1b3c6d) & m
+    return (h >> np.uint64(32 - log2cap)) >> np.uint64(3)
+
+
+@pytest.mark.parametrize("ksize", [(3, 3, 3), (5, 1, 3)])
+def test_full_buckets(ksize):
+    """As many groups as the table takes of one size (5456 of 8192 slots): about
+    one bucket in ten has more than eight and overflows into the next."""
+    n, spatial = 5456, (20, 30, 40)
+    rng = np.random.default_rng(1)
+    group = rng.choice(20 * 30 * 10, n, replace=False)
+    c = np.stack([np.zeros(n, np.int64), group // 300, group // 10 % 30, group % 10 * 4 + rng.integers(0, 4, n)], 1).astype(np.int32)
+    assert np.bincount(_bucket(group.astype(np.uint64), 13).astype(np.int64), minlength=1024).max() > 8
+    pt = build_pair_table(torch.from_numpy(c).cuda(), spatial, ksize=ksize)
+    pf, pb, _ = po.subm_pairs(c, spatial, ksize)
+    assert np.array_equal(pt.pairs_fwd.cpu().numpy(), pf)
+    assert np.array_equal(pt.pairs_bwd.cpu().numpy(), pb)
