@@ -18,6 +18,7 @@ oracle/pairs_oracle.py):
 * strided-conv outputs are numbered in ascending (batch, z, y, x) order.
 """
 import ctypes
+import weakref
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence
 
@@ -35,13 +36,14 @@ def _vp(t: torch.Tensor):
 
 
 _I32x3 = ctypes.c_int32 * 3
+_LO, _HI = -(1 << 31), (1 << 31) - 1
 
 
 def _i32x3(v: Sequence[int]):
     """The first three ints as a host array (an argument of the C entry
-    points).  ctypes would wrap a value that 32 bits do not hold."""
-    a, b, c = (int(x) for x in list(v)[:3])
-    if not all(-(1 << 31) <= x < 1 << 31 for x in (a, b, c)):
+    points).  ctypes wraps a value that 32 bits do not hold."""
+    a, b, c = map(int, v if len(v) == 3 else list(v)[:3])
+    if not (_LO <= a <= _HI and _LO <= b <= _HI and _LO <= c <= _HI):
         raise ValueError(f"{a}, {b}, {c}: a value does not fit 32 bits")
     return _I32x3(a, b, c)
 
@@ -86,16 +88,18 @@ class SpconvOps:
         # without a split the kernel writes the caller's mask row itself, where
         # that is n plain words beside the coordinates (else copy_ converts,
         # moves or refuses)
-        direct = (split_masks is None and masks.dtype == torch.int32 and masks.device == dev and
-                  tuple(masks[0].shape) == (n,) and masks[0].is_contiguous())
-        mask_full = masks[0] if direct else torch.empty(n, dtype=torch.int32, device=dev)
+        row = masks[0]
+        direct = (split_masks is None and row.dtype == torch.int32 and row.shape == (n,) and row.device == dev and
+                  row.is_contiguous())
+        mask_full = row if direct else torch.empty(n, dtype=torch.int32, device=dev)
         s = _stream(stream)
+        fwd = pairs.data_ptr() if n else None
+        bwd = fwd + 4 * pairs.stride(0) if n else None
         _lib.check(lib.sc_build_subm_pairs(
-            _vp(coords), n, sp, ks, dl, _vp(pairs[0]), _vp(pairs[1]), _vp(mask_full), _vp(ws),
-            ws.numel(), s))
+            _vp(coords), n, sp, ks, dl, fwd, bwd, _vp(mask_full), _vp(ws), ws.numel(), s))
         if split_masks is None:
             if not direct:
-                masks[0].copy_(mask_full)
+                row.copy_(mask_full)
         else:
             for j, sm in enumerate(split_masks):
                 masks[j].copy_(mask_full & _as_i32(sm))
@@ -173,16 +177,12 @@ class SpconvOps:
         ``mask``: the sorted masks [N], bit k (of the kv-bit reversed word with
         ``reverse``) set exactly where out[k][r] != -1; absent entries are then
         not read."""
-        _lib.require_cuda()
-        lib = _lib.load()
         ind, srt, msk = _t(indices), _t(argsort), _t(mask)
-        kv, n = ind.shape
+        n = ind.shape[1]
         if msk is not None and not (msk.numel() == n and msk.dtype in (torch.int32, torch.uint32) and
                                     msk.device == ind.device and msk.is_contiguous()):
             raise ValueError(f"mask must be {n} contiguous 32-bit words on the device of indices")
-        out = torch.empty_like(ind)
-        _lib.check(lib.sc_sort_indices_masked(_vp(ind), kv, n, _vp(srt), _vp(msk), 1 if reverse else 0,
-                                              _vp(out), _stream(stream)))
+        out = _sort_indices(ind, srt, msk, reverse, stream)
         if isinstance(indices, tv.Tensor):
             return tv.Tensor(out, tv.int32)
         return out
@@ -210,14 +210,28 @@ class SpconvOps:
         return out
 
 
+def _sort_indices(ind: torch.Tensor, order: torch.Tensor, mask, reverse: bool, stream: int) -> torch.Tensor:
+    """sort_indices of a mask that fits."""
+    _lib.require_cuda()
+    kv, n = ind.shape
+    out = torch.empty_like(ind)
+    _lib.check(_lib.load().sc_sort_indices_masked(_vp(ind), kv, n, _vp(order), _vp(mask), 1 if reverse else 0,
+                                                  _vp(out), _stream(stream)))
+    return out
+
+
 def _as_i32(v: int) -> int:
     v &= 0xffffffff
     return v - (1 << 32) if v >= (1 << 31) else v
 
 
-def _version(t: torch.Tensor):
-    """Count of torch's writes to t (inference tensors keep none)."""
-    return None if t.is_inference() else t._version
+def _versions(tensors):
+    """torch's counts of the writes to the tensors (None: inference tensors, or
+    a table that the caller dropped)."""
+    try:
+        return [t._version for t in tensors]
+    except (RuntimeError, AttributeError):
+        return None
 
 
 @dataclass
@@ -242,30 +256,27 @@ class PairTable:
         """P = number of valid (input, output) pairs."""
         return int((self.pairs_fwd >= 0).sum().item())
 
-    def __setattr__(self, name, value):
-        if name in self.__dataclass_fields__:
-            self.__dict__.pop("_built", None)  # see _mark_built
-        object.__setattr__(self, name, value)
+    def _tables(self):
+        return (self.pairs_fwd, self.pairs_bwd, *self.masks_fwd, *self.argsorts_fwd, *self.masks_bwd,
+                *self.argsorts_bwd)
 
     def _mark_built(self):
         """Notes that the masks name exactly the pairs of the tables, in their
-        argsort's order, as the builder leaves them.  A table or list that is
-        assigned, a mask or argsort that is replaced, and a tensor that is
-        written through torch end that."""
-        rows = self.masks_fwd + self.argsorts_fwd + self.masks_bwd + self.argsorts_bwd
-        self.__dict__["_built"] = (rows, [_version(t) for t in self._tables_and_rows()])
+        argsort's order, as the builder leaves them.  Another tensor in their
+        place, and a write to one through torch (inference tensors do not
+        count those), end that."""
+        tables = self._tables()
+        self._built = [*map(weakref.ref, tables)], _versions(tables)
 
-    def _tables_and_rows(self):
-        return [self.pairs_fwd, self.pairs_bwd, *self.masks_fwd, *self.argsorts_fwd, *self.masks_bwd,
-                *self.argsorts_bwd]
-
-    def _masks_exact(self) -> bool:
-        if "_built" not in self.__dict__:
+    def _as_built(self) -> bool:
+        built = self.__dict__.get("_built")
+        if built is None:
             return False
-        rows, versions = self.__dict__["_built"]
-        now = self._tables_and_rows()
-        return (len(now) == len(versions) and all(a is b for a, b in zip(now[2:], rows)) and
-                [_version(t) for t in now] == versions)
+        tables = self._tables()
+        return [id(r()) for r in built[0]] == [*map(id, tables)] and _versions(tables) == built[1]
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_built"}
 
     def sorted_indices(self, which: str = "fwd", split: int = 0) -> torch.Tensor:
         """Index table of `which` ('fwd' or 'bwd') permuted into the argsort
@@ -276,15 +287,13 @@ class PairTable:
         cache = self.__dict__.setdefault("_sorted_cache", {})
         key = (which, split)
         if key not in cache:
-            back = self.argsorts_fwd if self.subm else self.argsorts_bwd
-            pairs, order = ((self.pairs_fwd, self.argsorts_fwd) if which == "fwd" else (self.pairs_bwd, back))
+            fwd, subm = which == "fwd", self.subm
+            pairs = self.pairs_fwd if fwd else self.pairs_bwd
+            order = (self.argsorts_fwd if fwd or subm else self.argsorts_bwd)[split]
             # the masks that the builder left say which entries exist; others
             # may disagree with the tables
-            mask = None
-            if self._masks_exact():
-                mask = (self.masks_fwd if which == "fwd" or self.subm else self.masks_bwd)[split]
-            cache[key] = SpconvOps.sort_indices(pairs, order[split], mask=mask,
-                                                reverse=which != "fwd" and self.subm)
+            mask = (self.masks_fwd if fwd or subm else self.masks_bwd)[split] if self._as_built() else None
+            cache[key] = _sort_indices(pairs, order, mask, not fwd and subm, 0)
         return cache[key]
 
     def tile_order(self, which: str = "fwd", split: int = 0) -> torch.Tensor:

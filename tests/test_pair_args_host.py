@@ -1,6 +1,7 @@
 """Host side of the pair builder's calls, with the native library replaced by a
 recorder: which addresses a call hands over, and what it refuses before that."""
 import dataclasses
+import pickle
 
 import numpy as np
 import pytest
@@ -117,7 +118,13 @@ def test_built_tables_are_sorted_by_their_own_masks(lib, change):
     assert _sorted_with(lib, pt, "bwd") == pt.masks_fwd[0].data_ptr()
     change(pt.masks_fwd)
     assert _sorted_with(lib, pt, "fwd") is None
-    # a copy with other masks is a table made by the caller
+    # the forward's table without the backward's
+    pt = build_pair_table(coords, (4, 4, 4))
+    pt.pairs_bwd = None
+    assert _sorted_with(lib, pt, "fwd") is None
+    # a copy with other masks is a table made by the caller, and a copy of the
+    # tensors is not what the builder left
+    assert _sorted_with(lib, pickle.loads(pickle.dumps(build_pair_table(coords, (4, 4, 4)))), "fwd") is None
     pt = build_pair_table(coords, (4, 4, 4))
     assert _sorted_with(lib, dataclasses.replace(pt, masks_fwd=[pt.masks_fwd[0] & 1]), "fwd") is None
 
