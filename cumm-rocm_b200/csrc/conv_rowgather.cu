@@ -83,7 +83,7 @@ struct Meta {
 };
 
 struct KParams {
-  CUtensorMap tmap_a;  // gathered rows [a_rows, red] (single layout)
+  CUtensorMap tmap_a;  // gathered rows [a_rows, red] (gather path)
   CUtensorMap tmap_b;  // B rows [n_total, kv * red] (TMA path)
   // four rows of zeros with tmap_a's box and swizzle: a gather whose four
   // rows are all -1 reads these instead (out-of-range gather rows cost the
@@ -508,7 +508,7 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
           for (int q = 0; q < 4; ++q) {
             const int64_t rq = tile_m * kTileM + q * 32 + lane;
             uint32_t v = rq < A.M ? (A.mask ? __ldg(A.mask + rq) : 1u) : 0u;
-    v = __reduce_or_sync(0xffffffffu, v);
+            v = __reduce_or_sync(0xffffffffu, v);
             gq[q] = v;
           }
           g0 = gq[0];
@@ -591,13 +591,13 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
     const int pw = warp - kProdWarp0;
     if constexpr (kGather) {
     // Groups of P.group_warps warps take the chunks in turn, each warp an equal
-    // share of the rows: a chunk costs a warp a fixed ~1,000 cycles of waits and
-    // set-up beside its rows, so fewer warps per chunk and more chunks in
+    // share of the rows: a chunk costs a warp a fixed 700-1,000 cycles of waits
+    // and set-up beside its rows, so fewer warps per chunk and more chunks in
     // flight fill the ring faster.  There are at most as many groups as
     // stages: a group that tests stage s then knows the use before the last
     // one to be consumed, which the parity test needs.
     // TMA tile::gather4, one lane per four rows (an index of -1 is an
-    // out-of-range row and lands as zeros): about 130 cycles of a warp's issue
+    // out-of-range row and lands as zeros): 110-130 cycles of a warp's issue
     // each, asynchronous from there.  With all producer warps on every chunk,
     // against two: 60k voxels C = K = 128 forward 94 -> 62 us, C = K = 256
     // 191 -> 154; 200k voxels, stride 2, E4M3 64 -> 128 47 -> 39.  16-byte
@@ -965,7 +965,7 @@ __global__ void __maxnreg__(kPair ? 80 : 96)
 //
 // What bounds it, from clock64() counters of every role (200k voxels, C = K =
 // 64): not the tensor core (its warp waits) but the time a chunk holds its
-// stage: a gather4 takes ~110 cycles of its warp's issue, so ~1,750 for a
+// stage: a gather4 takes 110-130 cycles of its warp's issue, so 1,750-2,100 for a
 // warp's 16, then ~900 until the rows have landed, ~700 in the MMAs and ~500
 // until the stage is issued again, over 4 stages.  Hence two warps per chunk
 // and four chunks in flight.  Steps, forward us at 200k voxels / 2.6M voxels /
@@ -1126,8 +1126,8 @@ __global__ void __maxnreg__(72) conv_strand_kernel(const __grid_constant__ KPara
       // Groups of two warps take the strand's chunks in turn; a warp gathers
       // 64 rows of its group's chunk, lanes 0-15 one tile::gather4 each (four
       // sorted indices of the chunk's offset, gated by the row group's sub-tile
-      // mask; rows past M read as -1).  A gather4 takes about 130 cycles of a
-      // warp's issue and a chunk about 700 cycles of waits and set-up, so the
+      // mask; rows past M read as -1).  A gather4 takes 110-130 cycles of a
+      // warp's issue and a chunk 700-1,000 cycles of waits and set-up, so the
       // strand's rate is the chunks in flight over their sum.  The group's
       // first warp adds the weight slab.  A cursor runs one of the group's
       // chunks ahead of the one being issued and loads its indices.
@@ -1504,7 +1504,8 @@ cudaError_t launch_conv_rowgather(const ConvRowGatherArgs &a, int num_sms, cudaS
       P.num_tiles < (int64_t(1) << 30) && a.a_rows < (int64_t(1) << 31) && a.M < (int64_t(1) << 31) - 1024) {
     if (P.num_tiles == 0) return cudaSuccess;
     // Two CTAs per SM (113 KB each).  Two strands per CTA where every CTA has
-    // at least three tiles of one column block per offset; kernel us, one
+    // at least three tiles of one column block per offset, the least at which
+    // neither row width loses (64-byte rows alone gain from two); kernel us, one
     // strand / two: 128-byte rows 60k voxels (1.6 tiles) 26 / 30, 80k (2.1) 30 /
     // 31, 120k (3.2) 41 / 39, 200k 58.4 / 54.4, 300k 79 / 74, 2.6M 674 / 652;
     // 64-byte rows 40k (1.1) 18 / 25, 80k 28.0 / 26.5, 200k 55 / 48, 300k 76 /

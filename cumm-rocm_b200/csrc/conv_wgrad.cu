@@ -38,8 +38,8 @@ namespace {
 // CTAs per SM, 11 warps each, 80 registers; gather path with 64 dOut columns
 // and M-tile groups of <= 4 tiles = 256 TMEM columns): warps 0-3 epilogue,
 // 4-7 producers, 8-9 index loaders (one row, every filter of the group per
-// thread), 10 MMA; index tables of 8 filters.  The TMA gather rate is per
-// issuing CTA, so two CTAs on an SM gather faster than one.
+// thread), 10 MMA; index tables of 8 filters.  The gather rate goes with the
+// warps that issue and the stages they can fill, which two CTAs have more of.
 constexpr int kEpiWarps = 4;     // warps 0-3 in both layouts
 constexpr int kProdWarp0 = 4;
 template <bool kPair> struct Layout {

@@ -450,8 +450,8 @@ __device__ __forceinline__ void mma_commit_pair(uint64_t *bar) {
 // (M = 256, N = 256, K = 16) takes the 128 cycles of the single one's
 // M = 128.  Rank 0's MMA warp issues for both; its full barriers count both
 // CTAs' loads, and its commits release the stages of both.  The sums are the
-// single kernel's, in its order.  8192^3: 750 -> 686 us (1,600 TFLOP/s); what
-// is left is the tensor pipe at the clock that the power limit allows, and the
+// single kernel's, in its order.  8192^3 alone: 750 -> 686 us; after other work,
+// with L2 flushed, 724 (1,519 TFLOP/s; cuBLAS 679 in the same run).  What is left is the tensor pipe at the clock that the power limit allows, and the
 // last wave (1,024 units on 74 pairs: 13.8 waves).
 template <typename TOut>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)

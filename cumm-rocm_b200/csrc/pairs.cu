@@ -186,6 +186,7 @@ insert_groups(const int32_t *coords, int vec, int64_t n, Geom g, GroupTable t, i
 __device__ __forceinline__ void load_slot(const GroupSlot *s, unsigned long long &key, int4 &v) {
   unsigned long long pad, lo, hi;
   asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(key), "=l"(pad), "=l"(lo), "=l"(hi) : "l"(s));
+  (void)pad;
   v = make_int4(static_cast<int>(lo), static_cast<int>(lo >> 32), static_cast<int>(hi), static_cast<int>(hi >> 32));
 }
 
