@@ -113,6 +113,9 @@ struct GroupTable {
   int log2cap;
 };
 
+// Groups of a row of w >= 1 voxels (w + 3 may not fit an int).
+__device__ __forceinline__ int groups_of(int w) { return ((w - 1) >> 2) + 1; }
+
 // A 32-bit multiplicative hash of the folded key (neighbouring rows and groups
 // differ in its low bits, which the multiplications carry to the top): the top
 // bits name the slot that an insertion starts at, the low seven are the tag.
@@ -148,7 +151,7 @@ insert_groups(const int32_t *coords, int vec, int64_t n, Geom g, GroupTable t, i
   const bool in = i < n && c.x >= 0 && c.y >= 0 && c.z >= 0 && c.w >= 0 && c.y < g.spatial[0] &&
                   c.z < g.spatial[1] && c.w < g.spatial[2];
   if (i < n && !in) atomicOr(err, kErrBadIndex);
-  const int gsp[3] = {g.spatial[0], g.spatial[1], (g.spatial[2] + 3) >> 2};
+  const int gsp[3] = {g.spatial[0], g.spatial[1], groups_of(g.spatial[2])};
   const unsigned long long key = in ? static_cast<unsigned long long>(lin_key(c.x, c.y, c.z, c.w >> 2, gsp)) : ~0ull;
   const unsigned long long prev_key = __shfl_up_sync(0xffffffffu, key, 1);
   const bool leader = lane == 0 || prev_key != key;
@@ -235,7 +238,7 @@ subm_pairs_kernel(const int32_t *coords, int vec, int64_t n, Geom g, GroupTable 
   const bool live = i < n;
   const int4 co = live ? load_coord(coords, i, vec != 0) : make_int4(0, 0, 0, 0);
   const int z = co.y, y = co.z, x = co.w;
-  const int ng = (g.spatial[2] + 3) >> 2;
+  const int ng = groups_of(g.spatial[2]);
   const int gsp[3] = {g.spatial[0], g.spatial[1], ng};
   uint32_t m = 0;
   if constexpr (kNine) {

@@ -64,3 +64,15 @@ def test_full_buckets(ksize):
     pf, pb, _ = po.subm_pairs(c, spatial, ksize)
     assert np.array_equal(pt.pairs_fwd.cpu().numpy(), pf)
     assert np.array_equal(pt.pairs_bwd.cpu().numpy(), pb)
+
+
+@pytest.mark.parametrize("ksize", [(3, 3, 3), (1, 1, 5)])
+@pytest.mark.parametrize("width", [2 ** 31 - 1, 2 ** 31 - 3])
+def test_widest_rows(width, ksize):
+    """Rows as wide as int32 coordinates allow, voxels at both ends."""
+    x = np.concatenate([np.arange(6), width - 1 - np.arange(6)])
+    c = np.stack([np.zeros(24, np.int64), np.zeros(24, np.int64), np.repeat([0, 1], 12), np.tile(x, 2)], 1).astype(np.int32)
+    pt = build_pair_table(torch.from_numpy(c).cuda(), (1, 2, width), ksize=ksize)
+    pf, pb, _ = po.subm_pairs(c, (1, 2, width), ksize)
+    assert np.array_equal(pt.pairs_fwd.cpu().numpy(), pf)
+    assert np.array_equal(pt.pairs_bwd.cpu().numpy(), pb)
