@@ -270,16 +270,18 @@ __device__ __forceinline__ void epilogue_cols(const KParams &P, float *acc, int6
   const EpiParams &e = P.a.epi;
   const bool use_src = e.beta != 0.f && e.src != nullptr;
   if (e.mode == 1) {
-    if (e.scale != nullptr) {
-#pragma unroll
-      for (int i = 0; i < n; ++i) acc[i] = __ldg(e.scale + col + i) * acc[i];
-    }
+    // scale * acc + alpha * bias, the product and the sum rounded together
+    float bias[n];
     if (e.bias != nullptr) {
-      float bias[n];
       load_src<n, TOut>(reinterpret_cast<const TOut *>(e.bias) + col, bias);
 #pragma unroll
-      for (int i = 0; i < n; ++i) acc[i] = acc[i] + e.alpha * bias[i];
+      for (int i = 0; i < n; ++i) bias[i] *= e.alpha;
+    } else {
+#pragma unroll
+      for (int i = 0; i < n; ++i) bias[i] = 0.f;
     }
+#pragma unroll
+    for (int i = 0; i < n; ++i) acc[i] = fmaf(e.scale != nullptr ? __ldg(e.scale + col + i) : 1.f, acc[i], bias[i]);
   } else {
 #pragma unroll
     for (int i = 0; i < n; ++i) acc[i] = e.alpha * acc[i];
